@@ -322,3 +322,35 @@ def test_sampling_with_history_penalties_matches_the_oracle(ctx, oracle, shape):
     # the plain entry point refuses what it cannot apply
     with pytest.raises(tsb.TsbError):
         ctx.sample(ctx.to_device(lg), ctx.to_device(unis), batch, vocab, cfg, toks, margins, ctx.alloc(ctx.accept_scratch_bytes(batch, 1, vocab)))
+
+
+@pytest.mark.parametrize("vocab,batch", [(2, 3), (9, 40), (1023, 8), (8191, 30), (65537, 9), (131070, 2), (131071, 4), (163840, 2)])
+@pytest.mark.parametrize("kind", ["ties", "masked", "constant"])
+def test_rows_counted_by_value_match_the_oracle(ctx, oracle, vocab, batch, kind):
+    """Vocabularies at the edges of the statistics kernel's slices (rows that start off a 16-byte boundary, clusters of two, four and
+    eight, more than 65535 entries of one value), values that tie across a cut, rows masked with the type's lowest value."""
+    rng = np.random.default_rng(vocab + batch)
+    k = 2
+    tgt = np.round(rng.standard_normal((batch, k + 1, vocab)) * 2.0).astype(np.float32) / 2  # ties: a few dozen values, both signs of zero
+    if kind == "masked":
+        tgt[:, :, rng.permutation(vocab)[: vocab - 1 - vocab // 3]] = -65504.0
+    elif kind == "constant":
+        tgt[:] = -1.5
+    drf = np.roll(tgt[:, :k], 1, axis=2)
+    t16, d16 = oracle.f32_to_f16_bits(tgt), oracle.f32_to_f16_bits(drf)
+    checked = 0
+    for shape in (dict(temperature=1.0), dict(temperature=0.0), dict(temperature=0.7, top_p=0.8), dict(temperature=1.3, top_k=7, min_p=0.2),
+                  dict(temperature=1.0, top_k=200, top_p=0.95)):
+        ocfg = oracle.shaping(seed=4, **shape)
+        props = rng.integers(0, vocab, size=(batch, k)).astype(np.int32)
+        unis = rng.integers(0, 2**63, size=(batch, 2 * k + 1)).astype(np.uint64) * np.uint64(2)
+        outs = _run_accept(ctx, oracle, t16, d16, props, unis, **shape)
+        for b in range(min(batch, 3)):
+            acc, toks, draws, margins = oracle.accept_round(t16[b], d16[b], props[b], ocfg, unis[b])
+            # equal probabilities are the rule here, so r * q <= p is often decided within rounding: such rounds say nothing
+            if shape["temperature"] and (margins[0] < 1e-12 or margins[1] < 1e-12):
+                continue
+            checked += 1
+            assert outs[b].status == 0 and outs[b].accepted == acc and outs[b].draws == draws, (shape, b)
+            assert list(outs[b].tokens[:acc + 1]) == list(toks), (shape, b, list(outs[b].tokens[:acc + 1]), list(toks))
+    assert checked > 0
