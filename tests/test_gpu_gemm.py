@@ -338,3 +338,30 @@ def test_a_wait_nobody_answers_gives_up_reports_and_leaves_the_context_usable(or
                oracle.gemm_quant(0, q, rows, cols, oracle.f16_bits_to_f32(x16)))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("rows,cols,tokens", [(6144, 4096, 33), (6144, 4096, 64), (6144, 4096, 65), (6144, 4096, 96), (6144, 4096, 112), (4096, 14336, 128),
+                                              (19072, 512, 80), (19072, 512, 257)])
+def test_the_tensor_memory_path_repeats_its_bits_over_weights_that_come_from_memory(ctx, rows, cols, tokens):
+    """Launches back to back over more weights than the L2 cache holds, where copies arrive late and stages are refilled while the
+    tensor core keeps shared memory busy: every launch gives the bits of the same product computed on its own.  Widths on both
+    sides of the lines where the kernel's rings and accumulator copies change (64, 96, 128 token rows)."""
+    from turbospark_b200 import opbench
+    rng = np.random.default_rng(rows + tokens)
+    w_bytes = rows * cols // 256 * 144
+    ws = [ctx.upload_weights(opbench.random_blocks("q4k", rows, cols, rng)) for _ in range(max(3, int(2.2 * (126 << 20)) // w_bytes))]
+    xd = ctx.to_device(rng.standard_normal((tokens, cols)).astype(np.float16).view(np.uint16))
+    ys = [ctx.alloc(tokens * rows * 4) for _ in ws]
+    alone = []
+    for w, y in zip(ws, ys):
+        ctx.gemm_quant(0, w, rows, cols, xd, y, tokens, y_f32=True)
+        ctx.sync()
+        alone.append(y.download(np.uint32, tokens * rows))
+    for _ in range(4):
+        for w, y in zip(ws, ys):
+            ctx.gemm_quant(0, w, rows, cols, xd, y, tokens, y_f32=True)
+        ctx.sync()
+        for y, want in zip(ys, alone):
+            assert np.array_equal(y.download(np.uint32, tokens * rows), want)
+    for b in ws + ys + [xd]:
+        b.free()
