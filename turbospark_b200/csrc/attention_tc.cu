@@ -1,9 +1,8 @@
 // Split-KV attention for passes with many queries per (stream, kv head) - a speculative tree's 65 rows x the head
 // group, or a prefill chunk - on the fifth-generation tensor cores.  head_dim 128.
 //
-// A CTA owns one (stream, kv head, 128-query tile, KV chunk) and walks the chunk in 128-token tiles (one
-// tcgen05.mma costs about a hundred cycles however narrow it is: 94 with both operands in shared memory and N <= 128,
-// 111 with A in tensor memory, 128 = the full rate only at N = 256 - so the tiles are as wide as tensor memory allows):
+// A CTA owns one (stream, kv head, 128-query tile, KV chunk) and walks the chunk in 128-token tiles, as wide as tensor
+// memory allows:
 //   warps 0-7  two softmax warpgroups.  Thread t of group w is query t of the tile - it owns lane t of tensor memory -
 //              and takes tokens 64 w .. 64 w + 63 of every tile: it reads its half row of S = Q K^T (tcgen05.ld),
 //              applies the tree mask, meets the other group's half-row maximum through shared memory, and writes
@@ -190,62 +189,62 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             if (!ok) bars->failed = 1;
         }
     } else if (warp == TC_SOFTMAX_WARPS + TC_LOAD_WARPS) {
-        // ---- MMA issue: the warp walks the tiles together, lane 0 issues
-        const uint32_t leader = lane == 0 ? 1u : 0u;
-        // instruction descriptors: f32 accumulate, f16 A and B, M = 128; scores N = 128 tokens, both operands K-major;
-        // P V N = 128 columns with B (V) MN-major
-        const uint32_t idesc_s = (1u << 4) | ((uint32_t)(TC_TN >> 3) << 17) | ((uint32_t)(TC_QM >> 4) << 24);
-        const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(TC_HD >> 3) << 17) | ((uint32_t)(TC_QM >> 4) << 24);
-        // shared-memory matrix descriptors without the start address (version 1, 128-byte swizzle).  K-major (Q, K):
-        // eight-row groups 1024 bytes apart (stride byte offset), the leading offset is not used; a K = 16 step moves
-        // the start address by 32 bytes inside the 64-element block, the second block starts rows * 128 bytes later.
-        // MN-major (V): eight-token groups 1024 bytes apart (stride), the two 64-column blocks a block's size apart (leading)
-        constexpr uint64_t SW128 = 2ull << 61;
-        const uint64_t desc_kmaj = ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | SW128;
-        const uint64_t desc_mnmaj = ((uint64_t)((uint32_t)(TC_TN * 128) >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | SW128;
-        const uint64_t desc_q = desc_kmaj | (uint64_t)((smem_u32(q_tile) >> 4) & 0x3FFFu);
-        bool ok = true;
-        auto scores = [&](int t) {  // S(t) into accumulator t & 1
-            const int st = t % TC_STAGES;
-            ok = mbar_wait(&bars->kv_full[st], (t / TC_STAGES) & 1, err);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) return;
-            tc_fence_after();
-            const uint64_t desc_k = desc_kmaj | (uint64_t)((smem_u32(ring + st * TC_STAGE_BYTES) >> 4) & 0x3FFFu);
-            const uint32_t d = tmem + TC_COL_S + (uint32_t)(t & 1) * TC_TN;
-            tc_mma_ss<false>(leader, d, desc_q, desc_k, idesc_s);
+        // ---- MMA issue: one thread walks the tiles
+        if (tc_elect()) {
+            // instruction descriptors: f32 accumulate, f16 A and B, M = 128; scores N = 128 tokens, both operands K-major;
+            // P V N = 128 columns with B (V) MN-major
+            const uint32_t idesc_s = (1u << 4) | ((uint32_t)(TC_TN >> 3) << 17) | ((uint32_t)(TC_QM >> 4) << 24);
+            const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(TC_HD >> 3) << 17) | ((uint32_t)(TC_QM >> 4) << 24);
+            // shared-memory matrix descriptors without the start address (version 1, 128-byte swizzle).  K-major (Q, K):
+            // eight-row groups 1024 bytes apart (stride byte offset), the leading offset is not used; a K = 16 step moves
+            // the start address by 32 bytes inside the 64-element block, the second block starts rows * 128 bytes later.
+            // MN-major (V): eight-token groups 1024 bytes apart (stride), the two 64-column blocks a block's size apart (leading)
+            constexpr uint64_t SW128 = 2ull << 61;
+            const uint64_t desc_kmaj = ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | SW128;
+            const uint64_t desc_mnmaj = ((uint64_t)((uint32_t)(TC_TN * 128) >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | SW128;
+            const uint64_t desc_q = desc_kmaj | (uint64_t)((smem_u32(q_tile) >> 4) & 0x3FFFu);
+            bool ok = true;
+            auto scores = [&](int t) {  // S(t) into accumulator t & 1
+                const int st = t % TC_STAGES;
+                ok = mbar_wait(&bars->kv_full[st], (t / TC_STAGES) & 1, err);
+                if (!ok) return;
+                tc_fence_after();
+                const uint64_t desc_k = desc_kmaj | (uint64_t)((smem_u32(ring + st * TC_STAGE_BYTES) >> 4) & 0x3FFFu);
+                const uint32_t d = tmem + TC_COL_S + (uint32_t)(t & 1) * TC_TN;
+                tc_issue_ss<false>(d, desc_q, desc_k, idesc_s);
 #pragma unroll
-            for (int ks = 1; ks < TC_HD / 16; ks++) {  // address units of 16 bytes: 32 bytes per step, a block per four steps
-                const uint32_t in_block = (uint32_t)(ks & 3) * 2u;
-                tc_mma_ss<true>(leader, d, desc_q + (uint64_t)((uint32_t)(ks >> 2) * (TC_QM * 128 / 16) + in_block),
-                                desc_k + (uint64_t)((uint32_t)(ks >> 2) * (TC_TN * 128 / 16) + in_block), idesc_s);
+                for (int ks = 1; ks < TC_HD / 16; ks++) {  // address units of 16 bytes: 32 bytes per step, a block per four steps
+                    const uint32_t in_block = (uint32_t)(ks & 3) * 2u;
+                    tc_issue_ss<true>(d, desc_q + (uint64_t)((uint32_t)(ks >> 2) * (TC_QM * 128 / 16) + in_block),
+                                      desc_k + (uint64_t)((uint32_t)(ks >> 2) * (TC_TN * 128 / 16) + in_block), idesc_s);
+                }
+                tc_commit(&bars->s_full[t & 1]);
+            };
+            if (n_tiles > 0) scores(0);
+            if (ok && n_tiles > 1) scores(1);
+            for (int t = 0; t < n_tiles && ok; t++) {
+                const int st = t % TC_STAGES;
+                ok = mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, err);
+                if (!ok) break;
+                TTRC(t, 1);
+                tc_fence_after();
+                const uint64_t desc_v = desc_mnmaj | (uint64_t)((smem_u32(ring + st * TC_STAGE_BYTES + TC_TILE_BYTES) >> 4) & 0x3FFFu);
+                const uint32_t d = tmem + TC_COL_PV;
+                const uint32_t a = tmem + TC_COL_S + (uint32_t)(t & 1) * TC_TN;  // P sits where the tile's scores were
+                if (t == 0) tc_issue_ts<false>(d, a, desc_v, idesc_pv);  // the first tile starts the output
+                else tc_issue_ts<true>(d, a, desc_v, idesc_pv);
+#pragma unroll
+                for (int kt = 1; kt < TC_TN / 16; kt++)  // sixteen tokens per step: two 1024-byte token groups = 128 address units
+                    tc_issue_ts<true>(d, a + 8 * kt, desc_v + (uint64_t)(128 * kt), idesc_pv);
+                tc_commit(&bars->pv_full);
+                tc_commit(&bars->kv_empty[st]);
+                TTRC(t, 0);
+                if (t + 2 < n_tiles) scores(t + 2);
+                TTRC(t, 2);
             }
-            tc_commit_if(leader, &bars->s_full[t & 1]);
-        };
-        if (n_tiles > 0) scores(0);
-        if (ok && n_tiles > 1) scores(1);
-        for (int t = 0; t < n_tiles && ok; t++) {
-            const int st = t % TC_STAGES;
-            ok = mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, err);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            TTRC(t, 1);
-            tc_fence_after();
-            const uint64_t desc_v = desc_mnmaj | (uint64_t)((smem_u32(ring + st * TC_STAGE_BYTES + TC_TILE_BYTES) >> 4) & 0x3FFFu);
-            const uint32_t d = tmem + TC_COL_PV;
-            const uint32_t a = tmem + TC_COL_S + (uint32_t)(t & 1) * TC_TN;  // P sits where the tile's scores were
-            if (t == 0) tc_mma_ts<false>(leader, d, a, desc_v, idesc_pv);  // the first tile starts the output
-            else tc_mma_ts<true>(leader, d, a, desc_v, idesc_pv);
-#pragma unroll
-            for (int kt = 1; kt < TC_TN / 16; kt++)  // sixteen tokens per step: two 1024-byte token groups = 128 address units
-                tc_mma_ts<true>(leader, d, a + 8 * kt, desc_v + (uint64_t)(128 * kt), idesc_pv);
-            tc_commit_if(leader, &bars->pv_full);
-            tc_commit_if(leader, &bars->kv_empty[st]);
-            TTRC(t, 0);
-            if (t + 2 < n_tiles) scores(t + 2);
-            TTRC(t, 2);
+            if (!ok) bars->failed = 1;
         }
-        if (!ok && lane == 0) bars->failed = 1;
+        __syncwarp();
     } else {
         // ---- softmax warpgroups: thread = (query ql of the tile = tensor-memory lane ql, half wg of every tile's 128 tokens).
         // A failed wait does not leave the loop: the other group's barriers still get their arrivals, nobody is left waiting.

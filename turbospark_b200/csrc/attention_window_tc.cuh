@@ -184,8 +184,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1)
             // no copy is in flight when the CTA leaves, also when another role has given up
             for (int t = lane > 0 ? issued : issued > WT_STAGES ? issued - WT_STAGES : 0; t < issued; t++) mbar_wait(&bars->kv_full[t % WT_STAGES], (t / WT_STAGES) & 1, err);
         }
-        if (warp == 9) {
-            const uint32_t leader = lane == 0 ? 1u : 0u;
+        if (warp == 9 && tc_elect()) {  // MMA issue: one thread walks the tiles
             // f32 accumulate, bfloat16 operands, M = 128; scores: N = TN tokens, both operands K-major; output: N = DV, B MN-major
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(WT_QM >> 4) << 24);
             const uint32_t idesc_s = idesc | ((uint32_t)(WT_TN >> 3) << 17), idesc_o = idesc | (1u << 16) | ((uint32_t)(DV >> 3) << 17);
@@ -197,17 +196,17 @@ __global__ void __launch_bounds__(WT_THREADS, 1)
                 const uint64_t dq = kmaj | (uint64_t)((smem_u32(q_tiles + x * QTILE) >> 4) & 0x3FFFu);
                 const uint64_t dk = kmaj | (uint64_t)((smem_u32(ring + (t % WT_STAGES) * STAGE) >> 4) & 0x3FFFu);
                 const uint32_t d = tmem + WT_COL_S + (uint32_t)x * 128;
-                tc_mma_ss<false>(leader, d, dq, dk, idesc_s);
+                tc_issue_ss<false>(d, dq, dk, idesc_s);
 #pragma unroll
                 for (int ks = 1; ks < DK / 16; ks++) {
                     const uint64_t step = (uint64_t)((uint32_t)(ks & 3) * 2u);
-                    tc_mma_ss<true>(leader, d, dq + (uint64_t)((uint32_t)(ks >> 2) * (128 * 128 / 16)) + step,
-                                    dk + (uint64_t)((uint32_t)(ks >> 2) * (WT_TN * 128 / 16)) + step, idesc_s);
+                    tc_issue_ss<true>(d, dq + (uint64_t)((uint32_t)(ks >> 2) * (128 * 128 / 16)) + step,
+                                      dk + (uint64_t)((uint32_t)(ks >> 2) * (WT_TN * 128 / 16)) + step, idesc_s);
                 }
-                tc_commit_if(leader, &bars->s_full[x]);
+                tc_commit(&bars->s_full[x]);
             };
             if (n_tiles > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&bars->kv_full[0], 0u, err));
+                ok = mbar_wait(&bars->kv_full[0], 0u, err);
                 tc_fence_after();
                 for (int x = 0; x < n_wg && ok; x++) scores(x, 0);
             }
@@ -215,27 +214,28 @@ __global__ void __launch_bounds__(WT_THREADS, 1)
                 const int st = t % WT_STAGES;
                 const uint64_t dv = mnmaj | (uint64_t)((smem_u32(ring + st * STAGE + Geo::V_AT) >> 4) & 0x3FFFu);
                 for (int x = 0; x < n_wg && ok; x++) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(&bars->p_full[x], t & 1, err));
+                    ok = mbar_wait(&bars->p_full[x], t & 1, err);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t d = tmem + WT_COL_O + (uint32_t)x * DV, p = tmem + WT_COL_S + (uint32_t)x * 128;  // P lies over the scores
-                    if (t == 0) tc_mma_ts<false>(leader, d, p, dv, idesc_o);
-                    else tc_mma_ts<true>(leader, d, p, dv, idesc_o);
+                    if (t == 0) tc_issue_ts<false>(d, p, dv, idesc_o);
+                    else tc_issue_ts<true>(d, p, dv, idesc_o);
 #pragma unroll
-                    for (int kt = 1; kt < WT_TN / 16; kt++) tc_mma_ts<true>(leader, d, p + 8 * kt, dv + (uint64_t)(128 * kt), idesc_o);
-                    if (x == n_wg - 1) tc_commit_if(leader, &bars->kv_empty[st]);
+                    for (int kt = 1; kt < WT_TN / 16; kt++) tc_issue_ts<true>(d, p + 8 * kt, dv + (uint64_t)(128 * kt), idesc_o);
+                    if (x == n_wg - 1) tc_commit(&bars->kv_empty[st]);
                     if (t + 1 < n_tiles) {
                         if (x == 0) {
-                            ok = __all_sync(0xffffffffu, mbar_wait(&bars->kv_full[(t + 1) % WT_STAGES], ((t + 1) / WT_STAGES) & 1, err));
+                            ok = mbar_wait(&bars->kv_full[(t + 1) % WT_STAGES], ((t + 1) / WT_STAGES) & 1, err);
                             tc_fence_after();
                         }
                         if (ok) scores(x, t + 1);  // in order behind the product that reads P from the same columns
                     } else {
-                        tc_commit_if(leader, &bars->o_full[x]);
+                        tc_commit(&bars->o_full[x]);
                     }
                 }
             }
         }
+        __syncwarp();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WT_REGS_LARGE));
         if (warp / 4 < n_wg) {

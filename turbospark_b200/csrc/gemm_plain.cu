@@ -609,39 +609,41 @@ __global__ void __launch_bounds__(TCG_THREADS, 1)
             for (uint32_t k = it > (uint32_t)stages ? it - stages : 0; k < it; k++) mbar_wait(&bars->full[k % stages], (k / stages) & 1, err);
         }
     } else if (warp == TCG_EPI_WARPS + 1) {
-        // ---- MMA issue: the warp walks the items together, lane 0 issues.  f32 accumulate, bfloat16 operands, both
+        // ---- MMA issue: one thread walks the items.  f32 accumulate, bfloat16 operands, both
         // K-major and 128-byte swizzled (eight-row groups 1024 bytes apart; a K = 16 step moves the start by 32 bytes)
-        const uint32_t leader = lane == 0 ? 1u : 0u;
-        auto idesc_of = [](int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TCG_M >> 4) << 24); };
-        constexpr uint64_t DESC = ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-        bool ok = true;
-        uint32_t it = 0, tile = 0;
-        for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x, tile++) {
-            const Item w = item_of(i);
-            const uint32_t buf = tile & 1;
-            if (tile >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_empty[buf], ((tile >> 1) - 1) & 1, err));
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t d = tmem + buf * (uint32_t)nt;
-            // an expert's tile multiplies only the tokens it has
-            const uint32_t idesc = EXPERTS ? idesc_of(max(16, (w.n_tok + 15) & ~15)) : idesc_of(nt);
-            for (int u = 0; u < w.n; u++, it++) {
-                const int s = it % stages;
-                ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], (it / stages) & 1, err));
+        if (tc_elect()) {
+            auto idesc_of = [](int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TCG_M >> 4) << 24); };
+            constexpr uint64_t DESC = ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+            bool ok = true;
+            uint32_t it = 0, tile = 0;
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x, tile++) {
+                const Item w = item_of(i);
+                const uint32_t buf = tile & 1;
+                if (tile >= 2) ok = mbar_wait(&bars->acc_empty[buf], ((tile >> 1) - 1) & 1, err);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_addr = smem_u32(ring + s * stage_bytes);
-                const uint64_t da = DESC | (uint64_t)((a_addr >> 4) & 0x3FFFu);
-                const uint64_t db = DESC | (uint64_t)(((a_addr + TCG_M * 128) >> 4) & 0x3FFFu);
-                if (u == 0) tc_mma_ss<false>(leader, d, da, db, idesc);
-                else tc_mma_ss<true>(leader, d, da, db, idesc);
+                const uint32_t d = tmem + buf * (uint32_t)nt;
+                // an expert's tile multiplies only the tokens it has
+                const uint32_t idesc = EXPERTS ? idesc_of(max(16, (w.n_tok + 15) & ~15)) : idesc_of(nt);
+                for (int u = 0; u < w.n; u++, it++) {
+                    const int s = it % stages;
+                    ok = mbar_wait(&bars->full[s], (it / stages) & 1, err);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(ring + s * stage_bytes);
+                    const uint64_t da = DESC | (uint64_t)((a_addr >> 4) & 0x3FFFu);
+                    const uint64_t db = DESC | (uint64_t)(((a_addr + TCG_M * 128) >> 4) & 0x3FFFu);
+                    if (u == 0) tc_issue_ss<false>(d, da, db, idesc);
+                    else tc_issue_ss<true>(d, da, db, idesc);
 #pragma unroll
-                for (int ks = 1; ks < TCG_K / 16; ks++) tc_mma_ss<true>(leader, d, da + 2u * ks, db + 2u * ks, idesc);
-                tc_commit_if(leader, &bars->empty[s]);
+                    for (int ks = 1; ks < TCG_K / 16; ks++) tc_issue_ss<true>(d, da + 2u * ks, db + 2u * ks, idesc);
+                    tc_commit(&bars->empty[s]);
+                }
+                if (ok) tc_commit(&bars->acc_full[buf]);
             }
-            if (ok) tc_commit_if(leader, &bars->acc_full[buf]);
+            if (!ok) bars->failed = 1;
         }
-        if (!ok && lane == 0) bars->failed = 1;
+        __syncwarp();
     } else {
         // ---- epilogue: two threads per weight row of the tile, columns = tokens.  One destination per tile and thread, one short
         // loop per kind of destination: the code of a kind has to stay in the instruction cache.

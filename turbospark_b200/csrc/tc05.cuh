@@ -11,36 +11,9 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// D[tmem_d] (+)= A[tmem_a] * B[smem descriptor]; M = 128, K = 16, f16 inputs, f32 accumulate.  ACC = false overwrites D.
-// The whole MMA warp runs the issue loop in step and only the instruction itself is predicated on `leader`: addresses
-// and descriptors are then warp-uniform values, and the issuing warp - which shares its scheduler with other warps of
-// the CTA - spends as few instructions per MMA as possible.
-template <bool ACC>
-__device__ __forceinline__ void tc_mma_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, e;\n"
-        "setp.ne.b32 e, %5, 0;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "r"(idesc), "n"(ACC ? 1 : 0), "r"(leader)
-        : "memory");
-}
-// the same with A from shared memory (a matrix descriptor like B's)
-template <bool ACC>
-__device__ __forceinline__ void tc_mma_ss(uint32_t leader, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, e;\n"
-        "setp.ne.b32 e, %5, 0;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(ACC ? 1 : 0), "r"(leader)
-        : "memory");
-}
-// One lane of a converged warp, always the same one.  A thread that this picks issues the three below on its own: an MMA whose
+// D[tmem_d] (+)= A[tmem_a] * B[smem descriptor]; M = 128, K = 16, f16 or bfloat16 inputs, f32 accumulate.  ACC = false overwrites D.
+// tc_issue_ss: A from shared memory (a matrix descriptor like B's).
+// One lane of a converged warp, always the same one.  A thread that this picks issues the instructions and the commits on its own: an MMA whose
 // predicate differs between the lanes of a converged warp took 75 to 90 cycles to issue, one from a single thread about 25.
 __device__ __forceinline__ bool tc_elect() {
     uint32_t one;
@@ -73,16 +46,6 @@ __device__ __forceinline__ void tc_issue_ss(uint32_t tmem_d, uint64_t desc_a, ui
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
         "}\n" ::"r"(tmem_d),
         "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(ACC ? 1 : 0)
-        : "memory");
-}
-__device__ __forceinline__ void tc_commit_if(uint32_t leader, uint64_t* bar) {
-    asm volatile(
-        "{\n"
-        ".reg .pred e;\n"
-        "setp.ne.b32 e, %1, 0;\n"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-        "}\n" ::"r"(smem_u32(bar)),
-        "r"(leader)
         : "memory");
 }
 // generic-proxy writes to shared memory become visible to the tensor core's (async-proxy) reads
