@@ -759,3 +759,23 @@ def test_a_model_loaded_from_a_resident_weight_file_gives_the_same_logits(oracle
     with pytest.raises(tsb.TsbError, match="dtype tag"):
         resident.ResidentIndex(bad).load_into(tsb.Model(ctx, cfg))
     idx.close(), direct.close(), loaded.close(), wrong.close(), ctx.close()
+
+
+@pytest.mark.parametrize("n", [2, 64, 65, 66, 130, 300])
+def test_prompts_in_one_pass_match_the_oracle_and_the_same_prompt_in_portions(rig, oracle, n):
+    """The many-row path takes a prompt's rows in one pass, in groups of 64 that see one another as committed rows: the token behind
+    the prompt matches the oracle, and so does a prompt whose second half arrives in a pass of its own."""
+    tsb = rig["tsb"]
+    rng = np.random.default_rng(n)
+    prompt = rng.integers(0, rig["cfg"].vocab, size=n + 1).astype(np.int32)
+    want = oracle.State(rig["ot"]).forward(prompt, 0)[n]
+    once = tsb.run_config(tsb.shaping(temperature=0.0), 1, 1)
+    sess = tsb.Session(rig["ctx"], rig["target"], None, 1, 32)
+    sess.sequential_run(prompt[:n], once)
+    _close(oracle, sess.produce(int(prompt[n]), n), want, rel=4e-3, abs_=4e-3)
+    half = n // 2 + 1
+    sess.reset()
+    sess.sequential_run(prompt[:half], once)
+    sess.sequential_run(prompt[:n], tsb.run_config(tsb.shaping(temperature=0.0), 1, 1, reuse_prefix=True))
+    _close(oracle, sess.produce(int(prompt[n]), n), want, rel=4e-3, abs_=4e-3)
+    sess.close()

@@ -744,10 +744,11 @@ template <int HD, int MT>
 static cudaError_t launch_attn_t(tsb_ctx* ctx, cudaStream_t st, const AttnPlan& p, dim3 grid, size_t smem, KvView view, int layer,
                                  const __half* q, int64_t q_stride, const tsb_row_desc* rows_dev, int rows_per_seq,
                                  int n_q_heads, float scale_log2e, float* part_o, float2* part_ml, uint32_t* tickets,
-                                 __half* out, ActOut act, int defer_merge = 0) {
+                                 __half* out, ActOut act, int defer_merge = 0, bool prompt = false) {
     static SmemOptIn configured;
     if (cudaError_t e = tsb_opt_in_smem(ctx, attn_partial_kernel<HD, MT>, smem, configured); e != cudaSuccess) return e;
-    return tsb_launch_cluster(ctx, attn_partial_kernel<HD, MT>, grid, dim3(ATT_THREADS * MT), smem, st, true,
+    // the kernel reads cache rows before it waits for its predecessor: without that licence it starts after it
+    return tsb_launch_cluster(ctx, attn_partial_kernel<HD, MT>, grid, dim3(ATT_THREADS * MT), smem, st, !prompt,
                               (unsigned)p.cluster_size, view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads,
                               scale_log2e, p.chunk, p.cluster_size, part_o, part_ml, tickets, out, act, ctx->dev_error, defer_merge);
 }
@@ -780,7 +781,7 @@ static cudaError_t launch_attn_merge(tsb_ctx* ctx, cudaStream_t st, const float*
 
 cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                     __half* out, ActOut act, const tsb_row_desc* rows_dev, int rows, int rows_per_seq,
-                                    int n_q_heads, float scale, int max_len, void* scratch, int rows_cap) {
+                                    int n_q_heads, float scale, int max_len, void* scratch, int rows_cap, bool prompt) {
     if (attn_split_merge_mode()) {
         // every chunk CTA leaves its share in memory and a second, wide launch merges them (one CTA per row and head)
         const float* part_o;
@@ -790,12 +791,12 @@ cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, i
             // many queries per (stream, kv head), or streams enough to fill the device: the tensor-memory kernel; its shares
             // always go through the merge
             cudaError_t e = launch_attn_tc_partials(ctx, st, kv, layer, q, q_stride, rows_dev, rows, rows_per_seq, n_q_heads, scale, max_len,
-                                                    scratch, &part_o, &part_ml, &n_splits);
+                                                    scratch, &part_o, &part_ml, &n_splits, prompt);
             if (e != cudaSuccess) return e;
             return launch_attn_merge(ctx, st, part_o, part_ml, n_splits, rows, n_q_heads, kv->view.head_dim, out, act);
         }
         cudaError_t e = launch_attn_partials(ctx, st, kv, layer, q, q_stride, rows_dev, rows, rows_per_seq, n_q_heads, scale, max_len, scratch,
-                                             &part_o, &part_ml, &n_splits, out, act);
+                                             &part_o, &part_ml, &n_splits, out, act, prompt);
         if (e != cudaSuccess || n_splits == 1) return e;  // a single split wrote the output itself
         return launch_attn_merge(ctx, st, part_o, part_ml, n_splits, rows, n_q_heads, kv->view.head_dim, out, act);
     }
@@ -813,15 +814,15 @@ cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, i
     if (hd == 128) {
         if (p.mt == 2)
             return launch_attn_t<128, 2>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads,
-                                         scale_log2e, part_o, part_ml, tickets, out, act);
+                                         scale_log2e, part_o, part_ml, tickets, out, act, 0, prompt);
         return launch_attn_t<128, 1>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads,
-                                     scale_log2e, part_o, part_ml, tickets, out, act);
+                                     scale_log2e, part_o, part_ml, tickets, out, act, 0, prompt);
     }
     if (p.mt == 2)
         return launch_attn_t<64, 2>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads,
-                                    scale_log2e, part_o, part_ml, tickets, out, act);
+                                    scale_log2e, part_o, part_ml, tickets, out, act, 0, prompt);
     return launch_attn_t<64, 1>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads,
-                                scale_log2e, part_o, part_ml, tickets, out, act);
+                                scale_log2e, part_o, part_ml, tickets, out, act, 0, prompt);
 }
 
 // The split plan of the partials-only launch: no clusters, as many KV chunks per (stream, kv head, query tile) as
@@ -829,7 +830,7 @@ cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, i
 // CTA every K/V byte of a chunk is in flight from the first instruction.  Like attn_plan it is made for the length rounded up
 // to 512 and does not depend on the row count while the queries fit one tile, so a row gets the same chunks - and
 // the same sums - whether it is verified in a batch or decoded alone.
-static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len) {
+static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, bool prompt) {
     AttnPlan p;
     const int G = n_q_heads / kv->view.kv_heads;
     const int n_queries = rows_per_seq * G;
@@ -839,6 +840,10 @@ static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int row
     p.n_qtiles = (n_queries + 16 * p.mt - 1) / (16 * p.mt);
     p.groups = rows / rows_per_seq;
     p.cluster_size = 1;
+    if (prompt) {
+        p.chunk = attn_prompt_chunk(max_len), p.n_splits = attn_prompt_splits(max_len);
+        return p;
+    }
     const int planned = max_len > 0 ? (max_len + 511) / 512 * 512 : 512;
     const int tiles_total = planned / TILE_TOKENS;
     const int base_ctas = p.groups * kv->view.kv_heads * p.n_qtiles;
@@ -874,8 +879,8 @@ extern "C" __attribute__((visibility("default"))) void tsb_debug_set_attn_trace(
 cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                  const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int n_q_heads, float scale, int max_len,
                                  void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, __half* out_single,
-                                 ActOut act_single) {
-    const AttnPlan p = attn_plan_partials(ctx, kv, rows, rows_per_seq, n_q_heads, max_len);
+                                 ActOut act_single, bool prompt) {
+    const AttnPlan p = attn_plan_partials(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt);
     const int hd = kv->view.head_dim;
     float* part_o = reinterpret_cast<float*>(scratch);
     float2* part_ml = reinterpret_cast<float2*>(part_o + (size_t)rows * n_q_heads * p.n_splits * hd);
@@ -892,7 +897,7 @@ cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int 
     const int defer = single ? 0 : 1;
 #define TSB_ATTN_LAUNCH(HDV, MTV)                                                                                                          \
     return launch_attn_t<HDV, MTV>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads, scale_log2e, part_o, \
-                                   part_ml, ATTN_TICKETS, out, act, defer)
+                                   part_ml, ATTN_TICKETS, out, act, defer, prompt)
     if (hd == 128) {
         if (p.mt == 4) TSB_ATTN_LAUNCH(128, 4);
         if (p.mt == 2) TSB_ATTN_LAUNCH(128, 2);
@@ -903,6 +908,8 @@ cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int 
     TSB_ATTN_LAUNCH(64, 1);
 #undef TSB_ATTN_LAUNCH
 }
+
+int attn_prompt_splits(int max_len) { return attn_split_merge_mode() ? (max_len + attn_prompt_chunk(max_len) - 1) / attn_prompt_chunk(max_len) : MAX_SPLITS; }
 
 extern "C" {
 

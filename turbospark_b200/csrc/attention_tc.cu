@@ -405,11 +405,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 struct TcPlan {
     int n_qtiles, groups, n_splits, chunk;
 };
-TcPlan attn_tc_plan(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len) {
+TcPlan attn_tc_plan(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, bool prompt) {
     TcPlan p;
     const int G = n_q_heads / kv->view.kv_heads;
     p.n_qtiles = (rows_per_seq * G + TC_QM - 1) / TC_QM;
     p.groups = rows / rows_per_seq;
+    if (prompt) {
+        p.chunk = attn_prompt_chunk(max_len), p.n_splits = attn_prompt_splits(max_len);
+        return p;
+    }
     const int planned = max_len > 0 ? (max_len + 511) / 512 * 512 : 512;
     const int tiles_total = planned / TC_TN;
     const int base_ctas = p.groups * kv->view.kv_heads * p.n_qtiles;
@@ -501,8 +505,8 @@ bool attn_tc_applicable(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows
 
 cudaError_t launch_attn_tc_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                     const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int n_q_heads, float scale, int max_len,
-                                    void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out) {
-    const TcPlan p = attn_tc_plan(ctx, kv, rows, rows_per_seq, n_q_heads, max_len);
+                                    void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, bool prompt) {
+    const TcPlan p = attn_tc_plan(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt);
     float* part_o = reinterpret_cast<float*>(scratch);
     float2* part_ml = reinterpret_cast<float2*>(part_o + (size_t)rows * n_q_heads * p.n_splits * TC_HD);
     *part_o_out = part_o, *part_ml_out = part_ml, *n_splits_out = p.n_splits;

@@ -96,9 +96,8 @@ __global__ void __launch_bounds__(256) wide_prepare_kernel(const __half* __restr
     pdl_wait();
     const int blk = blockIdx.x;
     const int pass = blockIdx.y / (per_pass >> 3), grp = blockIdx.y % (per_pass >> 3);
-    const int nt = min(per_pass, tokens - pass * per_pass);  // token rows of this pass
-    const int n_pad = (nt + 15) / 16 * 16;
-    if (nt <= 0 || grp * 8 >= n_pad) return;
+    const int nt = min(per_pass, tokens - pass * per_pass);  // token rows of this pass; the others are zeros
+    const int n_pad = per_pass;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = grp * 8 + w;  // token row within the pass
     uint4 o = make_uint4(0, 0, 0, 0);
@@ -146,18 +145,22 @@ __device__ __forceinline__ void tensor_g2s_2d(void* dst_smem, const CUtensorMap*
 // WIDE_LAUNCH_REGS), which launch_gemm_wide_q4k checks against the compiled kernel: the increase waits until the others
 // have given theirs up.
 constexpr int WIDE_LAUNCH_REGS = 96;
-constexpr int WIDE_REGS_FEED = 64, WIDE_REGS_DEQ = 80, WIDE_REGS_FOLD = 128;
-static_assert(WIDE_REGS_FEED + 2 * WIDE_REGS_DEQ + 2 * WIDE_REGS_FOLD <= WIDE_THREADS / 128 * WIDE_LAUNCH_REGS, "register shares");
+template <bool MANY>
+struct WideRegs {
+    static constexpr int FEED = MANY ? 32 : 64, DEQ = MANY ? 72 : 80, FOLD = MANY ? 152 : 128;
+    static_assert(FEED + 2 * DEQ + 2 * FOLD <= WIDE_THREADS / 128 * WIDE_LAUNCH_REGS, "register shares");
+};
 template <int N>
 __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
 __device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// ROUNDS: how many 16-column read-backs cover a warp's share of the accumulator columns (n_pad / 2 <= 16 * ROUNDS)
-template <int ROUNDS>
+// ROUNDS: how many 16-column read-backs cover a warp's share of the accumulator columns (n_pad / 2 <= 16 * ROUNDS).
+// MANY: several passes of n_pad token rows in one launch (see launch_gemm_wide_q4k)
+template <int ROUNDS, bool MANY>
 __global__ void __launch_bounds__(WIDE_THREADS, 1)
     gemm_wide_q4k_kernel(const __grid_constant__ CUtensorMap wmap, int64_t rows, int units, const uint4* __restrict__ xw, int n_pad,
-                         int tokens, void* __restrict__ y, int64_t y_stride, int y_f32, int n_whole, int ksplit, float* __restrict__ part,
+                         int all_tokens, int passes, void* __restrict__ y, int64_t y_stride, int y_f32, int n_whole, int ksplit, float* __restrict__ part,
                          uint32_t* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     WideBars* bars = reinterpret_cast<WideBars*>(smem);
@@ -176,15 +179,21 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     // remaining tiles - fewer than CTAs - is cut into `ksplit` runs of its blocks so that the last wave fills the
     // device too.  A run leaves its partial sums in `part` (after 1024 ticket words); the CTA that finishes a tile's last
     // run adds them in run order and writes the tile.
+    // MANY: an item is a whole tile for one of the passes, the passes of a tile side by side so that its weights come from
+    // memory once; the runs of a tile that a single pass would cut are added in the same order, in registers.
     const int n_tiles = (int)(rows / WM);
-    const int n_items = n_whole + (n_tiles - n_whole) * ksplit;
+    const int n_items = MANY ? n_tiles * passes : n_whole + (n_tiles - n_whole) * ksplit;
     const int upk = (units + ksplit - 1) / ksplit;  // blocks per run
     struct Item {
         int tile, b0, nblk, ks;  // ks < 0: a whole tile
+        int pass;
     };
     auto item_of = [&](int item) {
         Item it;
-        if (item < n_whole) {
+        it.pass = 0;
+        if (MANY) {
+            it.tile = item / passes, it.pass = item % passes, it.b0 = 0, it.nblk = units, it.ks = -1;
+        } else if (item < n_whole) {
             it.tile = item, it.b0 = 0, it.nblk = units, it.ks = -1;
         } else {
             const int t = item - n_whole;
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     const uint32_t tmem_a = tmem_d1 + 2 * (uint32_t)n_pad;
 
     if (warp < 4) {
-        regs_give<WIDE_REGS_FEED>();
+        regs_give<WideRegs<MANY>::FEED>();
         if (warp == WIDE_WARP_RAW) {
             // ---- producer of the raw blocks: one tensor copy (128 rows x 144 bytes) per block.  Weights come from no
             // kernel that this launch may overlap, so the ring fills before the activations are there.
@@ -254,7 +263,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                         if (nb >= n_bst) ok = mbar_wait(&bars->b_empty[bs], ((nb / n_bst) - 1) & 1, err);
                         if (!ok) break;
                         mbar_expect_tx(&bars->b_full[bs], (uint32_t)b_stage_bytes);
-                        bulk_g2s(b_ring + bs * b_stride, xw + (size_t)(wi.b0 + blk) * WIDE_CHUNKS * n_pad, (uint32_t)b_stage_bytes, &bars->b_full[bs]);
+                        bulk_g2s(b_ring + bs * b_stride, xw + (size_t)(wi.pass * units + wi.b0 + blk) * WIDE_CHUNKS * n_pad, (uint32_t)b_stage_bytes, &bars->b_full[bs]);
                     }
                 }
                 if (!ok) bars->failed = 1;
@@ -311,7 +320,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         }
     } else if (warp < 12) {
         // ---- dequantisation: a warpgroup takes one half (sub-blocks 4h .. 4h + 3) of every block, thread = row of the tile
-        regs_give<WIDE_REGS_DEQ>();
+        regs_give<WideRegs<MANY>::DEQ>();
         const int h = (warp >> 2) - 1, q4 = warp & 3;
         const int row = q4 * 32 + lane;
         const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         if (!ok && lane == 0) bars->failed = 1;
     } else {
         // ---- fold and epilogue: a warpgroup takes half of the token columns, thread = row of the tile
-        regs_take<WIDE_REGS_FOLD>();
+        regs_take<WideRegs<MANY>::FOLD>();
         const int g = (warp >> 2) - 3, q4 = warp & 3;
         const int row = q4 * 32 + lane;
         const int cpw = n_pad >> 1;
@@ -391,12 +400,34 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             const Item wi = item_of(item);
             const int nblk = wi.nblk, tile = wi.tile, ks = wi.ks;
-            float acc[16 * ROUNDS];
+            const bool runs = MANY && ksplit > 1 && tile >= n_whole;
+            int run_left = upk;
+            float acc[16 * ROUNDS], total[MANY ? 16 * ROUNDS : 1];
 #pragma unroll
             for (int i = 0; i < 16 * ROUNDS; i++) acc[i] = 0.f;
+            if (MANY) {
+#pragma unroll
+                for (int i = 0; i < 16 * ROUNDS; i++) total[i] = 0.f;
+            }
+            auto end_run = [&]() {
+#pragma unroll
+                for (int i = 0; i < 16 * ROUNDS; i++) total[MANY ? i : 0] += acc[i], acc[i] = 0.f;
+                run_left = upk;
+            };
             // acc += by * (this warp's share of an accumulator); 32 columns per round trip, columns past the share are read
             // and dropped
             auto fold = [&](uint32_t from, float by) {
+                if constexpr (MANY) {  // the sums of finished runs leave room for sixteen
+#pragma unroll
+                    for (int c = 0; c < ROUNDS; c++)
+                        if (16 * c < cpw) {
+                            uint32_t v[16];
+                            tc_ld16(from + col0 + 16 * c, v);
+                            tc_wait_ld(v);
+#pragma unroll
+                            for (int i = 0; i < 16; i++) acc[16 * c + i] = fmaf(by, __uint_as_float(v[i]), acc[16 * c + i]);
+                        }
+                } else {
 #pragma unroll
                 for (int c = 0; c < ROUNDS; c += 2)
                     if (16 * c < cpw) {
@@ -410,6 +441,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                             acc[16 * c + 16 + i] = fmaf(by, __uint_as_float(v1[i]), acc[16 * c + 16 + i]);
                         }
                     }
+                }
                 tc_fence_before();
                 __syncwarp();
             };
@@ -428,13 +460,20 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                 if (lane == 0) mbar_arrive(&bars->a_full[(nb + d2_sets) & 1][1]);
                 fold(tmem_d1 + set * (uint32_t)n_pad, d);
                 if (lane == 0) mbar_arrive(&bars->a_full[set][0]);
+                if (MANY && runs && --run_left == 0) end_run();
+            }
+            if (MANY && runs) {
+                if (run_left != upk) end_run();
+#pragma unroll
+                for (int i = 0; i < 16 * ROUNDS; i++) acc[i] = total[MANY ? i : 0];
             }
             const int64_t orow = (int64_t)tile * WM + row;
             // this thread's share of the token columns: cpw of them from n0 on, the ones behind the last token left out.
             // (Short code on purpose: unrolled over the accumulators, it runs once per tile out of a cold instruction cache.)
+            const int tok0 = MANY ? wi.pass * n_pad : 0, tokens = MANY ? min(n_pad, all_tokens - tok0) : all_tokens;
             const int n0 = g * cpw, n_mine = max(0, min(cpw, tokens - n0));
             auto put16 = [&](const float* v, int first) {  // sixteen columns from n0 + first on
-                const int64_t at = (int64_t)(n0 + first) * y_stride + orow;
+                const int64_t at = (int64_t)(tok0 + n0 + first) * y_stride + orow;
                 if (y_f32) {
                     float* p = reinterpret_cast<float*>(y) + at;
 #pragma unroll
@@ -447,7 +486,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                         if (first + i < n_mine) *p = __float2half_rn(v[i]);
                 }
             };
-            if (ks < 0) {
+            if (MANY || ks < 0) {
                 if (ok) {
 #pragma unroll
                     for (int c = 0; c < ROUNDS; c++) put16(acc + 16 * c, 16 * c);
@@ -547,6 +586,15 @@ static WidePlan wide_plan(int sm_count, int64_t rows, int units) {
     p.ksplit = (units + upk - 1) / upk;  // no empty runs: every run of a tile takes a ticket
     return p;
 }
+// Several passes in one launch when whole tiles of all of them fill the device about as well as one pass after the other with its
+// cut tiles does: the launch saves the passes' prologues and the traffic of their partial sums, and reads the weights once.
+static bool wide_takes_many(const WidePlan& p, int sm_count, int n_tiles, int units, int passes) {
+    if (passes < 2) return false;
+    const int tail = n_tiles - p.n_whole, upk = (units + p.ksplit - 1) / p.ksplit;
+    const int64_t one = (int64_t)p.n_whole / sm_count * units + (tail ? (int64_t)((tail * p.ksplit + sm_count - 1) / sm_count) * upk : 0) + (p.ksplit > 1 ? 5 : 1);
+    const int64_t many = ((int64_t)n_tiles * passes + sm_count - 1) / sm_count * units;
+    return many <= passes * one;
+}
 // the operand copy of every pass of a call with `tokens` token rows
 size_t gemm_wide_workspace_bytes(int64_t cols, int tokens) {
     const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX;
@@ -609,57 +657,58 @@ static cudaError_t wide_weight_map(const uint8_t* w, int64_t rows, int units, CU
 cudaError_t launch_gemm_wide_q4k(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t rows, int64_t cols, const __half* x,
                                  int64_t x_stride, int tokens, void* y, int64_t y_stride, bool y_f32, void* workspace, void* partials) {
     const int units = (int)(cols / 256);
-    static SmemOptIn configured1, configured2;
+    static SmemOptIn configured1, configured2, configured3;
     const size_t smem_max = std::max(wide_smem_bytes(WIDE_NDUAL), wide_smem_bytes(WIDE_NMAX));
-    if (cudaError_t e = tsb_opt_in_smem(ctx, gemm_wide_q4k_kernel<2>, smem_max, configured1); e != cudaSuccess) return e;
-    if (cudaError_t e = tsb_opt_in_smem(ctx, gemm_wide_q4k_kernel<4>, smem_max, configured2); e != cudaSuccess) return e;
+    if (cudaError_t e = tsb_opt_in_smem(ctx, gemm_wide_q4k_kernel<2, false>, smem_max, configured1); e != cudaSuccess) return e;
+    if (cudaError_t e = tsb_opt_in_smem(ctx, gemm_wide_q4k_kernel<4, false>, smem_max, configured2); e != cudaSuccess) return e;
+    if (cudaError_t e = tsb_opt_in_smem(ctx, gemm_wide_q4k_kernel<4, true>, smem_max, configured3); e != cudaSuccess) return e;
     static std::atomic<int> launch_regs{0};  // what the register shares are drawn on
     if (launch_regs.load() == 0) {
-        cudaFuncAttributes a1, a2;
-        if (cudaError_t e = cudaFuncGetAttributes(&a1, gemm_wide_q4k_kernel<2>); e != cudaSuccess) return e;
-        if (cudaError_t e = cudaFuncGetAttributes(&a2, gemm_wide_q4k_kernel<4>); e != cudaSuccess) return e;
-        launch_regs = std::min(a1.numRegs, a2.numRegs);
+        cudaFuncAttributes a1, a2, a3;
+        if (cudaError_t e = cudaFuncGetAttributes(&a1, gemm_wide_q4k_kernel<2, false>); e != cudaSuccess) return e;
+        if (cudaError_t e = cudaFuncGetAttributes(&a2, gemm_wide_q4k_kernel<4, false>); e != cudaSuccess) return e;
+        if (cudaError_t e = cudaFuncGetAttributes(&a3, gemm_wide_q4k_kernel<4, true>); e != cudaSuccess) return e;
+        launch_regs = std::min(a1.numRegs, std::min(a2.numRegs, a3.numRegs));
     }
     if (launch_regs.load() < WIDE_LAUNCH_REGS) return cudaErrorLaunchOutOfResources;
     CUtensorMap wmap;
     if (cudaError_t e = wide_weight_map(w, rows, units, &wmap); e != cudaSuccess) return e;
     // token rows go through in equal passes of at most WIDE_NMAX; one launch lays out the operand of every pass
     const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX;
-    const int per_pass = ((tokens + passes - 1) / passes + 15) / 16 * 16;
-    const size_t pass_chunks = (size_t)units * WIDE_CHUNKS * per_pass;
-    uint4* xw_all = static_cast<uint4*>(workspace);
+    const int n_pad = ((tokens + passes - 1) / passes + 15) / 16 * 16;
+    const size_t pass_chunks = (size_t)units * WIDE_CHUNKS * n_pad;
+    uint4* xw = static_cast<uint4*>(workspace);
     if (!workspace)
-        if (cudaError_t e = cudaMallocAsync((void**)&xw_all, pass_chunks * passes * 16, st); e != cudaSuccess) return e;
-    cudaError_t e = tsb_launch(ctx, wide_prepare_kernel, dim3((unsigned)units, (unsigned)(passes * (per_pass >> 3))), dim3(256), 0, st, true, x,
-                               x_stride, tokens, per_pass, units, xw_all);
-    for (int t0 = 0, pass = 0; t0 < tokens && e == cudaSuccess; t0 += per_pass, pass++) {
-        const int nt = min(per_pass, tokens - t0);
-        const int n_pad = (nt + 15) / 16 * 16;
-        const uint4* xw = xw_all + pass * pass_chunks;
-        const WidePlan plan = wide_plan(ctx->sm_count, rows, units);
-        const int ksplit = plan.ksplit;
-        if (e == cudaSuccess) {
-            // one CTA per SM: the kernel wants the whole tensor memory and most of the shared memory
-            const size_t smem = wide_smem_bytes(n_pad);
-            const int n_items = plan.n_whole + ((int)(rows / WM) - plan.n_whole) * ksplit;
-            dim3 grid((unsigned)min(n_items, ctx->sm_count));
-            uint8_t* yp = static_cast<uint8_t*>(y) + (size_t)t0 * y_stride * (y_f32 ? 4 : 2);
-            float* part = static_cast<float*>(partials);
-            if (ksplit > 1 && !part) {
-                e = cudaMallocAsync((void**)&part, 4096 + (size_t)ksplit * WIDE_NMAX * plan.tail_rows * sizeof(float), st);
-                if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, 4096, st);  // the ticket words start at zero
-            }
-            if (e == cudaSuccess) {
-                if (n_pad <= 64)
-                    e = tsb_launch(ctx, gemm_wide_q4k_kernel<2>, grid, dim3(WIDE_THREADS), smem, st, true, wmap, rows, units, (const uint4*)xw,
-                                   n_pad, nt, (void*)yp, y_stride, (int)(y_f32 ? 1 : 0), plan.n_whole, ksplit, part, ctx->dev_error);
-                else
-                    e = tsb_launch(ctx, gemm_wide_q4k_kernel<4>, grid, dim3(WIDE_THREADS), smem, st, true, wmap, rows, units, (const uint4*)xw,
-                                   n_pad, nt, (void*)yp, y_stride, (int)(y_f32 ? 1 : 0), plan.n_whole, ksplit, part, ctx->dev_error);
-            }
-            if (ksplit > 1 && !partials && part) cudaFreeAsync(part, st);
+        if (cudaError_t e = cudaMallocAsync((void**)&xw, pass_chunks * passes * 16, st); e != cudaSuccess) return e;
+    cudaError_t e = tsb_launch(ctx, wide_prepare_kernel, dim3((unsigned)units, (unsigned)(passes * (n_pad >> 3))), dim3(256), 0, st, true, x,
+                               x_stride, tokens, n_pad, units, xw);
+    const WidePlan plan = wide_plan(ctx->sm_count, rows, units);
+    const int n_tiles = (int)(rows / WM), ksplit = plan.ksplit;
+    const size_t smem = wide_smem_bytes(n_pad);
+    if (wide_takes_many(plan, ctx->sm_count, n_tiles, units, passes)) {
+        // one CTA per SM: the kernel wants the whole tensor memory and most of the shared memory
+        const dim3 grid((unsigned)min(n_tiles * passes, ctx->sm_count));
+        if (e == cudaSuccess)
+            e = tsb_launch(ctx, gemm_wide_q4k_kernel<4, true>, grid, dim3(WIDE_THREADS), smem, st, true, wmap, rows, units, (const uint4*)xw, n_pad, tokens, passes, y,
+                           y_stride, (int)(y_f32 ? 1 : 0), plan.n_whole, ksplit, (float*)nullptr, ctx->dev_error);
+    } else {
+        float* part = static_cast<float*>(partials);
+        const bool own_part = ksplit > 1 && !part;
+        if (own_part && e == cudaSuccess) {
+            e = cudaMallocAsync((void**)&part, 4096 + (size_t)ksplit * WIDE_NMAX * plan.tail_rows * sizeof(float), st);
+            if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, 4096, st);  // the ticket words start at zero
         }
+        const dim3 grid((unsigned)min(plan.n_whole + (n_tiles - plan.n_whole) * ksplit, ctx->sm_count));
+        for (int pass = 0; pass < passes && e == cudaSuccess; pass++) {
+            const int t0 = pass * n_pad, nt = min(n_pad, tokens - t0);
+            if (nt <= 0) break;
+            uint8_t* yp = static_cast<uint8_t*>(y) + (size_t)t0 * y_stride * (y_f32 ? 4 : 2);
+            auto kernel = n_pad <= WIDE_NDUAL ? gemm_wide_q4k_kernel<2, false> : gemm_wide_q4k_kernel<4, false>;
+            e = tsb_launch(ctx, kernel, grid, dim3(WIDE_THREADS), smem, st, true, wmap, rows, units, (const uint4*)(xw + pass * pass_chunks), n_pad, nt, 1, (void*)yp,
+                           y_stride, (int)(y_f32 ? 1 : 0), plan.n_whole, ksplit, part, ctx->dev_error);
+        }
+        if (own_part && part) cudaFreeAsync(part, st);
     }
-    if (!workspace) cudaFreeAsync(xw_all, st);
+    if (!workspace) cudaFreeAsync(xw, st);
     return e;
 }

@@ -215,7 +215,7 @@ int32_t tsb_session_create_pool(tsb_ctx* ctx, const tsb_model* target, const tsb
     if ((rc = A((size_t)n_streams * sizeof(int32_t), (void**)&s->tok1_dev))) return fail(rc);
     if ((rc = A((size_t)128 * 9 * sizeof(int32_t), (void**)&s->tree_dev))) return fail(rc);
     // pinned staging: descriptors and tokens of several forwards in flight
-    s->stage_cap = std::max(R * (2 * max_rows + 8), 2 * s->pass_rows);
+    s->stage_cap = std::max(std::max(R * (2 * max_rows + 8), 2 * s->pass_rows), 2 * s->target.prompt_rows);
     if (cudaMallocHost((void**)&s->stage_rows_host, (size_t)s->stage_cap * sizeof(tsb_row_desc)) != cudaSuccess) return fail(TSB_ERR_CUDA);
     if (cudaMallocHost((void**)&s->stage_tok_host, (size_t)s->stage_cap * sizeof(int32_t)) != cudaSuccess) return fail(TSB_ERR_CUDA);
     if ((rc = A((size_t)s->stage_cap * sizeof(tsb_row_desc), (void**)&s->stage_rows_dev))) return fail(rc);
@@ -978,12 +978,54 @@ int32_t session_ragged_pass(tsb_session* s, const RowGroup* groups, int n_groups
     return TSB_OK;
 }
 
+// A prompt's portion through a model that takes such passes: no head, cursor advanced.  Rows go in groups of PROMPT_GROUP, each
+// with the group's first position as its base (a row's mask covers its own group).
+static int32_t prompt_pass(tsb_session* s, ModelRt& rt, int stream, const int32_t* tokens, int n) {
+    tsb_ctx* ctx = s->ctx;
+    const int64_t pos = tsb_kv_cursor(rt.kv, stream);
+    if (pos + n > rt.model->cfg.max_context)
+        return tsb_fail(ctx, TSB_ERR_STATE, "stream %d: %lld + %d rows exceed the context window %d", stream, (long long)pos, n, rt.model->cfg.max_context);
+    int32_t rc = tsb_kv_reserve(rt.kv, stream, pos + n);
+    if (rc) return rc;
+    if (s->stage_used + n > s->stage_cap) {
+        TSB_CUDA(ctx, cudaStreamSynchronize(s->stream));
+        s->stage_used = 0;
+    }
+    tsb_row_desc* hd = s->stage_rows_host + s->stage_used;
+    int32_t* ht = s->stage_tok_host + s->stage_used;
+    for (int i = 0; i < n; i++) {
+        const int slot = i % PROMPT_GROUP;
+        tsb_row_desc& d = hd[i];
+        d.seq = stream, d.base = (int32_t)(pos + i - slot), d.slot = slot, d.position = (int32_t)(pos + i);
+        d.mask[0] = ~0ull >> (63 - slot), d.mask[1] = 0;
+        ht[i] = tokens[i];
+    }
+    Pass p;
+    p.rows_dev = s->stage_rows_dev + s->stage_used, p.tokens = s->stage_tok_dev + s->stage_used;
+    TSB_CUDA(ctx, cudaMemcpyAsync(s->stage_rows_dev + s->stage_used, hd, n * sizeof(tsb_row_desc), cudaMemcpyHostToDevice, s->stream));
+    TSB_CUDA(ctx, cudaMemcpyAsync(s->stage_tok_dev + s->stage_used, ht, n * sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
+    s->stage_used += n;
+    p.rows = n, p.rows_per_seq = n, p.max_len = (int)(pos + n), p.prompt = true;
+    record_fed(rt, stream, pos, tokens, n);
+    TSB_CUDA(ctx, rt.model->family->forward(s, rt, p));
+    tsb_kv_set_cursor(rt.kv, stream, pos + n);
+    return TSB_OK;
+}
+
 int32_t session_prefill_rows(tsb_session* s, int stream, const int32_t* tokens, int n) {
     TSB_REQUIRE(s->ctx, stream >= 0 && stream < s->n_streams, "stream %d outside the session", stream);
     if (s->target.model->family->ragged) {  // portions as large as a pass may be
         for (int i = 0; i < n; i += s->pass_rows) {
             const RowGroup g{stream, 0, std::min(s->pass_rows, n - i), tsb_kv_cursor(s->target.kv, stream)};
             int32_t rc = session_ragged_pass(s, &g, 1, tokens + i, g.n_rows, nullptr, 0);
+            if (rc) return rc;
+        }
+        return TSB_OK;
+    }
+    if (s->target.prompt_rows > 0) {
+        for (int i = 0, m; i < n; i += m) {
+            m = std::min(s->target.prompt_rows, n - i);
+            int32_t rc = prompt_pass(s, s->target, stream, tokens + i, m);
             if (rc) return rc;
         }
         return TSB_OK;

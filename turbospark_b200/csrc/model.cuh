@@ -80,6 +80,8 @@ struct ModelRt {
     ActBuf act_d, act_o, act_f;  // matmul operands of width d_model, n_q_heads*head_dim, ffn
     void* attn_scratch = nullptr;
     size_t attn_scratch_bytes = 0;
+    int attn_rows = 0;  // rows that scratch was sized for
+    int prompt_rows = 0;  // rows one pass over a prompt may carry on the tensor-memory path; 0: the family or the path has no such passes
     // wide_ok: every pass of this model in this session runs the tensor-memory matmul (all matrices Q4_K and the model's
     // largest pass has 24 rows or more) with natural-layout f16 buffers around it; otherwise every pass runs the
     // register path.  Never a mix: the two sum in different orders.
@@ -168,6 +170,7 @@ struct Pass {
     int64_t logits_stride = 0;
     bool last_rows_only = false;      // uniform passes: logits of each stream's last row only, one output row per stream
     int only = 0;                     // PASS_*
+    bool prompt = false;              // consecutive rows of one stream, in groups of PROMPT_GROUP (the last may be shorter) whose bases follow one another
     // ragged passes (families with `ragged`)
     const struct RowGroup* groups = nullptr;  // host
     int n_groups = 0;
@@ -176,6 +179,7 @@ struct Pass {
 };
 // Which launches of a pass are enqueued: all of them, or - for the two timing entry points - only the layer matmuls /
 // everything but the layer matmuls.
+constexpr int PROMPT_GROUP = 64;
 enum { PASS_ALL = 0, PASS_MATMULS = 1, PASS_REST = 2 };
 struct RowGroup {  // the rows of one stream in a ragged pass
     int seq, first_row, n_rows;

@@ -427,6 +427,7 @@ static int64_t blocks_weight_bytes(const tsb_model* m) {
     return t;
 }
 
+constexpr int PROMPT_ROWS = 1024;
 constexpr int WIDE_MIN_ROWS = 24;  // a model whose largest pass has this many rows or more runs every pass on the tensor-memory matmul
 
 static int32_t blocks_complete(const tsb_model* m) {
@@ -457,7 +458,25 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
                                shape.pages_per_seq, &rt.kv);
     if (rc) return rc;
     auto A = [&](size_t bytes, void** p) { return dev_alloc(ctx, s->owned, bytes, p); };
-    if ((rc = A((size_t)R * c.d_model * 2, (void**)&rt.h))) return rc;
+    // One matmul path per (session, model), whatever a pass's row count: the register path and the tensor-memory path
+    // sum in different orders, so a model that switched between them by row count would not reproduce its own
+    // single-row results in a batch (the reference's verify runs the decode path's arithmetic).  The tensor-memory path
+    // is taken when the model's largest pass has WIDE_MIN_ROWS rows or more: the target's verify carries max_rows rows
+    // of every stream; the drafter's largest pass is two rows per stream (a round's first step) or one stream's tree.
+    const int largest_pass = is_draft ? std::max(2 * n_streams, max_rows) : R;
+    bool wide = model->n_experts == 0 && largest_pass >= WIDE_MIN_ROWS && gemm_wide_supported(model->lm_head.qtype, model->lm_head.rows, model->lm_head.cols, R);
+    for (const LayerW& l : model->layers)
+        wide = wide && !l.wv.data && gemm_wide_supported(l.wqkv.qtype, l.wqkv.rows, l.wqkv.cols, R) && gemm_wide_supported(l.wo.qtype, l.wo.rows, l.wo.cols, R) &&
+               gemm_wide_supported(l.wgu.qtype, l.wgu.rows, l.wgu.cols, R) && gemm_wide_supported(l.wdown.qtype, l.wdown.rows, l.wdown.cols, R);
+    {
+        const char* env = getenv("TSB_WIDE_FORWARD");
+        if (env && env[0] == '0') wide = false;
+    }
+    // Prompts go through the target in passes of up to PROMPT_ROWS rows there: 1000 tokens of the 8B shape took 71 ms in passes of
+    // 64, whose weights are read and dequantised sixteen times.  Buffers of a pass: 170 MB at that shape.
+    if (wide && !is_draft) rt.prompt_rows = std::max(R, std::min(PROMPT_ROWS, c.max_context));
+    const int W = std::max(R, rt.prompt_rows);  // rows of the buffers a prompt's pass uses
+    if ((rc = A((size_t)W * c.d_model * 2, (void**)&rt.h))) return rc;
     if ((rc = A((size_t)R * c.n_q_heads * c.head_dim * 2, (void**)&rt.q))) return rc;
     if ((rc = A((size_t)R * c.head_dim * sizeof(float), (void**)&rt.cs))) return rc;
     if ((rc = A((size_t)(2 * c.n_layers + 1) * R * (c.d_model / 16) * sizeof(float), (void**)&rt.ss))) return rc;
@@ -471,7 +490,8 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
     cudaMemset(rt.act_d.xs, 0, act_xs_bytes(Rp, c.d_model));
     cudaMemset(rt.act_o.xs, 0, act_xs_bytes(Rp, od));
     cudaMemset(rt.act_f.xs, 0, act_xs_bytes(Rp, c.ffn));
-    rt.attn_scratch_bytes = attn_scratch_bytes(R, c.n_q_heads, c.head_dim);
+    rt.attn_rows = rt.prompt_rows ? std::max(R, 128) : R;  // a prompt's rows attend group by group where their shares do not fit at once
+    rt.attn_scratch_bytes = attn_scratch_bytes(rt.attn_rows, c.n_q_heads, c.head_dim);
     if ((rc = A(rt.attn_scratch_bytes, &rt.attn_scratch))) return rc;
     cudaMemset(rt.attn_scratch, 0, rt.attn_scratch_bytes);  // the ticket words start at zero
     rt.fed.assign(n_streams, std::vector<int32_t>());
@@ -494,26 +514,12 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
         }
         return TSB_OK;
     }
-    // One matmul path per (session, model), whatever a pass's row count: the register path and the tensor-memory path
-    // sum in different orders, so a model that switched between them by row count would not reproduce its own
-    // single-row results in a batch (the reference's verify runs the decode path's arithmetic).  The tensor-memory path
-    // is taken when the model's largest pass has WIDE_MIN_ROWS rows or more: the target's verify carries max_rows rows
-    // of every stream; the drafter's largest pass is two rows per stream (a round's first step) or one stream's tree.
-    const int largest_pass = is_draft ? std::max(2 * n_streams, max_rows) : R;
-    bool wide = largest_pass >= WIDE_MIN_ROWS && gemm_wide_supported(model->lm_head.qtype, model->lm_head.rows, model->lm_head.cols, R);
-    for (const LayerW& l : model->layers)
-        wide = wide && !l.wv.data && gemm_wide_supported(l.wqkv.qtype, l.wqkv.rows, l.wqkv.cols, R) && gemm_wide_supported(l.wo.qtype, l.wo.rows, l.wo.cols, R) &&
-               gemm_wide_supported(l.wgu.qtype, l.wgu.rows, l.wgu.cols, R) && gemm_wide_supported(l.wdown.qtype, l.wdown.rows, l.wdown.cols, R);
-    {
-        const char* env = getenv("TSB_WIDE_FORWARD");
-        if (env && env[0] == '0') wide = false;
-    }
     if (wide) {
         const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.d_model, od), c.ffn);
-        if ((rc = A((size_t)R * c.d_model * 2, (void**)&rt.w_xn)) || (rc = A((size_t)R * qkv_dim * 2, (void**)&rt.w_qkv)) ||
-            (rc = A((size_t)R * od * 2, (void**)&rt.w_ao)) || (rc = A((size_t)R * c.d_model * 2, (void**)&rt.w_o)) ||
-            (rc = A((size_t)R * 2 * c.ffn * 2, (void**)&rt.w_gu)) || (rc = A((size_t)R * c.ffn * 2, (void**)&rt.w_a)) ||
-            (rc = A((size_t)R * c.vocab * 2, (void**)&rt.w_logits)) || (rc = A(gemm_wide_workspace_bytes(widest, R), &rt.w_ws)))
+        if ((rc = A((size_t)W * c.d_model * 2, (void**)&rt.w_xn)) || (rc = A((size_t)W * qkv_dim * 2, (void**)&rt.w_qkv)) ||
+            (rc = A((size_t)W * od * 2, (void**)&rt.w_ao)) || (rc = A((size_t)W * c.d_model * 2, (void**)&rt.w_o)) ||
+            (rc = A((size_t)W * 2 * c.ffn * 2, (void**)&rt.w_gu)) || (rc = A((size_t)W * c.ffn * 2, (void**)&rt.w_a)) ||
+            (rc = A((size_t)R * c.vocab * 2, (void**)&rt.w_logits)) || (rc = A(gemm_wide_workspace_bytes(widest, W), &rt.w_ws)))
             return rc;
         size_t part = gemm_wide_partial_bytes(ctx, model->lm_head.rows, model->lm_head.cols);
         for (const LayerW& l : model->layers)
@@ -530,12 +536,28 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
 // gate|up -> silu*up -> down -> residual; crates/runtime/src/families/llama/mod.rs:205-291).
 static cudaError_t forward_device_wide(tsb_session* s, ModelRt& rt, const int32_t* tokens_dev, int token_stride,
                                        const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int max_len, __half* logits,
-                                       int64_t logits_stride, bool last_rows_only) {
+                                       int64_t logits_stride, bool last_rows_only, bool prompt) {
     tsb_ctx* ctx = s->ctx;
     cudaStream_t st = s->stream;
     const tsb_model* m = rt.model;
     const tsb_model_config& c = m->cfg;
     const float scale = 1.0f / sqrtf((float)c.head_dim);
+    // A prompt's groups attend like streams of one pass - a group sees the ones before it as committed rows, which the launch before
+    // has just written - as many at a time as their shares fit the scratch; the last, shorter one on its own.
+    auto attend_prompt = [&](int L, int64_t od, int64_t qkv_dim) -> cudaError_t {
+        for (int r0 = 0; r0 < rows;) {
+            const int per = std::min(PROMPT_GROUP, rows - r0);
+            int groups = (rows - r0) / per;
+            auto shares = [&](int g) { return (int64_t)g * per * attn_prompt_splits(max_len); };
+            const int64_t room = (int64_t)(rt.attn_scratch_bytes / ((size_t)c.n_q_heads * (c.head_dim + 2) * sizeof(float)));
+            while (groups > 1 && shares(groups) > room) groups = (groups + 1) / 2;
+            cudaError_t e = launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv + r0 * qkv_dim, qkv_dim, rt.w_ao + r0 * od, ActOut{nullptr, nullptr}, rows_dev + r0,
+                                                    groups * per, per, c.n_q_heads, scale, max_len, rt.attn_scratch, rt.attn_rows, true);
+            if (e != cudaSuccess) return e;
+            r0 += groups * per;
+        }
+        return cudaSuccess;
+    };
     const int64_t od = (int64_t)c.n_q_heads * c.head_dim, qkv_dim = (int64_t)(c.n_q_heads + 2 * c.n_kv_heads) * c.head_dim;
     const ActOut none{nullptr, nullptr};
     cudaError_t e;
@@ -550,8 +572,11 @@ static cudaError_t forward_device_wide(tsb_session* s, ModelRt& rt, const int32_
         const LayerW& l = m->layers[L];
         FW(launch_gemm_wide_q4k(ctx, st, l.wqkv.data, l.wqkv.rows, l.wqkv.cols, rt.w_xn, c.d_model, rows, rt.w_qkv, qkv_dim, false, rt.w_ws, rt.w_part));
         FW(launch_rope_store_kv(ctx, st, rt.kv, L, rt.w_qkv, rows_dev, rows, c.n_q_heads, c.rope_theta));
-        FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv, qkv_dim, rt.w_ao, none, rows_dev, rows, rows_per_seq, c.n_q_heads, scale,
-                                   max_len, rt.attn_scratch, s->n_streams * s->max_rows));
+        if (prompt)
+            FW(attend_prompt(L, od, qkv_dim));
+        else
+            FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv, qkv_dim, rt.w_ao, none, rows_dev, rows, rows_per_seq, c.n_q_heads, scale,
+                                       max_len, rt.attn_scratch, rt.attn_rows));
         FW(launch_gemm_wide_q4k(ctx, st, l.wo.data, l.wo.rows, l.wo.cols, rt.w_ao, od, rows, rt.w_o, c.d_model, false, rt.w_ws, rt.w_part));
         FW(launch_rmsnorm_rows(ctx, st, rt.h, rt.w_o, l.ffn_norm, rt.w_xn, none, rows, c.d_model, c.rms_eps));
         FW(launch_gemm_wide_q4k(ctx, st, l.wgu.data, l.wgu.rows, l.wgu.cols, rt.w_xn, c.d_model, rows, rt.w_gu, 2 * (int64_t)c.ffn, false, rt.w_ws, rt.w_part));
@@ -617,7 +642,7 @@ static cudaError_t forward_device_moe(tsb_session* s, ModelRt& rt, const int32_t
             }
         }
         FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.q, qd, nullptr, out_o, rows_dev, rows, rows_per_seq, c.n_q_heads, scale,
-                                   max_len, rt.attn_scratch, s->n_streams * s->max_rows));
+                                   max_len, rt.attn_scratch, rt.attn_rows));
         if (comm_world(s->comm) > 1) {
             // tensor-parallel attention: this rank's o_proj holds its heads' columns; the f32 shares are summed over the
             // ranks, then rounded to f16 once, as the single projection is
@@ -656,14 +681,14 @@ static cudaError_t forward_device_moe(tsb_session* s, ModelRt& rt, const int32_t
 // already on the device.  Cursors are not touched here.
 static cudaError_t forward_device(tsb_session* s, ModelRt& rt, const int32_t* tokens_dev, int token_stride,
                                   const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int max_len, __half* logits,
-                                  int64_t logits_stride, bool last_rows_only = false, int only = PASS_ALL) {
+                                  int64_t logits_stride, bool last_rows_only = false, int only = PASS_ALL, bool prompt = false) {
     const bool matmuls_only = only == PASS_MATMULS, skip_matmuls = only == PASS_REST;
     if (rt.model->n_experts > 0)
         return forward_device_moe(s, rt, tokens_dev, token_stride, rows_dev, rows, rows_per_seq, (max_len + 511) / 512 * 512, logits,
                                   logits_stride, last_rows_only);
     if (rt.wide_ok && only == PASS_ALL)
         return forward_device_wide(s, rt, tokens_dev, token_stride, rows_dev, rows, rows_per_seq, (max_len + 511) / 512 * 512, logits,
-                                   logits_stride, last_rows_only);
+                                   logits_stride, last_rows_only, prompt);
     tsb_ctx* ctx = s->ctx;
     cudaStream_t st = s->stream;
     const tsb_model* m = rt.model;
@@ -702,7 +727,7 @@ static cudaError_t forward_device(tsb_session* s, ModelRt& rt, const int32_t* to
         }
         if (!matmuls_only)
             FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.q, (int64_t)c.n_q_heads * c.head_dim, nullptr, out_o, rows_dev, rows,
-                                       rows_per_seq, c.n_q_heads, scale, max_len, rt.attn_scratch, s->n_streams * s->max_rows));
+                                       rows_per_seq, c.n_q_heads, scale, max_len, rt.attn_scratch, rt.attn_rows));
         if (skip_matmuls) continue;
         {   // o_proj; epilogue: residual add, next operand f16(h * g_ffn), partial sums of h^2
             EpiArgs a;
@@ -739,7 +764,7 @@ static int32_t blocks_fill_context(tsb_session* s, ModelRt& rt, int stream, int6
 
 static cudaError_t blocks_forward(tsb_session* s, ModelRt& rt, const Pass& p) {
     return forward_device(s, rt, p.tokens, p.token_stride, p.rows_dev, p.rows, p.rows_per_seq, p.max_len, (__half*)p.logits.p, p.logits_stride,
-                          p.last_rows_only, p.only);
+                          p.last_rows_only, p.only, p.prompt);
 }
 
 const ModelFamily BLOCKS_FAMILY = {
