@@ -410,7 +410,7 @@ __global__ void __maxnreg__(128)
                 for (int i = 0; i < 8; i++) pp[i] = __float2half_rn(accv[i]);
                 *reinterpret_cast<uint4*>(out + (size_t)row * n_q_heads * HD + e0) = pk;
             }
-            if (act.xp) act_store8(accv, act.xp, act.xs, row, e0, (n_q_heads * HD) >> 8, active);
+            if (act.xp) act_store8(accv, act, row, e0, (n_q_heads * HD) >> 8, active);
         } else if (active) {  // this cluster's share goes to memory; the last CTA of all clusters finishes the job
             const size_t pi = ((size_t)row * n_q_heads + head) * n_clusters + cl;
             float4* po = reinterpret_cast<float4*>(part_o + pi * HD + part * 8);
@@ -478,7 +478,7 @@ __global__ void __maxnreg__(128)
             for (int i = 0; i < 8; i++) pp[i] = __float2half_rn(accv[i]);
             *reinterpret_cast<uint4*>(out + (size_t)row * n_q_heads * HD + e0) = pk;
         }
-        if (act.xp) act_store8(accv, act.xp, act.xs, row, e0, (n_q_heads * HD) >> 8, active);
+        if (act.xp) act_store8(accv, act, row, e0, (n_q_heads * HD) >> 8, active);
     }
     if (cluster_size > 1) cluster.barrier_wait();
 }
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(MERGE_THREADS)
         for (int i = 0; i < 8; i++) pp[i] = __float2half_rn(o[i]);
         *reinterpret_cast<uint4*>(out + (size_t)row * n_q_heads * head_dim + e0) = pk;
     }
-    if (act.xp) act_store8(o, act.xp, act.xs, row, active ? e0 : 0, (n_q_heads * head_dim) >> 8, active);
+    if (act.xp) act_store8(o, act, row, active ? e0 : 0, (n_q_heads * head_dim) >> 8, active);
 }
 
 // The same merge for at most four splits: a thread is (query row x head, eight-column part) and folds the query's
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(MERGE_THREADS)
         for (int i = 0; i < 8; i++) pp[i] = __float2half_rn(o[i]);
         *reinterpret_cast<uint4*>(out + (size_t)row * n_q_heads * HD + e0) = pk;
     }
-    if (act.xp) act_store8(o, act.xp, act.xs, row, e0, (n_q_heads * HD) >> 8, active);
+    if (act.xp) act_store8(o, act, row, e0, (n_q_heads * HD) >> 8, active);
 }
 
 }  // namespace

@@ -40,4 +40,7 @@ cudaError_t launch_attn_tc_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, i
                                     const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int n_q_heads, float scale, int max_len,
                                     void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, bool prompt = false);
 cudaError_t launch_rope_store_kv(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, __half* qkv,
-                                 const tsb_row_desc* rows_dev, int rows, int n_q_heads, float theta);
+                                 const tsb_row_desc* rows_dev, int rows, int n_q_heads, float theta,
+                                 const float* table = nullptr);
+// table [rows, head_dim]: the cosines, then the sines, of every row's position
+cudaError_t launch_rope_table(tsb_ctx* ctx, cudaStream_t st, const tsb_row_desc* rows_dev, int rows, int head_dim, float theta, float* table);

@@ -436,7 +436,7 @@ __global__ void act_prepare_kernel(const __half* __restrict__ x, int64_t x_strid
         }
     }
     pdl_launch_dependents();
-    act_store8(v, xp, xs, t, e0, cols >> 8, active);
+    act_store8(v, ActOut{xp, xs}, t, e0, cols >> 8, active);
 }
 
 }  // namespace

@@ -29,9 +29,11 @@ struct ActOperand {
     const uint4* xp;  // [tiles][cols/256][8][32]
     const uint4* xs;  // [tiles][cols/256][32]
 };
-struct ActOut {  // where a producer writes an operand (both null = do not)
+struct ActOut {  // where a producer writes an operand (xp null = does not)
     uint4* xp;
     uint4* xs;
+    int wide = 0;  // > 0: the many-row matmul's operand instead, in passes of that many token rows (wide_operand; xs is not used)
+    int row0 = 0;  // the operand's token row of the producer's row 0
 };
 
 inline int act_tiles(int tokens) { return (tokens + 7) / 8; }
@@ -127,6 +129,8 @@ bool gemm_wide_supported(int qtype, int64_t rows, int64_t cols, int tokens);
 size_t gemm_wide_workspace_bytes(int64_t cols, int tokens);
 size_t gemm_wide_partial_bytes_for(int sm_count, int64_t rows, int64_t cols);  // the same for a device with that many SMs
 size_t gemm_wide_partial_bytes(const tsb_ctx* ctx, int64_t rows, int64_t cols);
+// x == nullptr: the workspace holds the operand already, written through wide_operand(workspace, tokens).
+ActOut wide_operand(void* workspace, int tokens);
 cudaError_t launch_gemm_wide_q4k(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t rows, int64_t cols, const __half* x,
                                  int64_t x_stride, int tokens, void* y, int64_t y_stride, bool y_f32, void* workspace = nullptr,
                                  void* partials = nullptr);
@@ -156,6 +160,21 @@ __device__ __forceinline__ void act_store_sum16(uint4* xs, int t, int col16, int
     q[comp * 2 + pos] = hi;
     q[4 + comp * 2 + pos] = __float2half_rn(s - __half2float(hi));
 }
+// The many-row matmul's operand: for every pass of n_pad token rows and every 256-column block, four 64-column blocks of n_pad
+// rows x 128 bytes, each row's eight 16-byte chunks XORed with the row's index mod 8 (the tensor core's 128-byte swizzle), then
+// two chunks a row with the sums of the block's eight 32-column runs, each a (high, remainder) pair of halves.
+constexpr int WIDE_CHUNKS = 34;
+__device__ __forceinline__ void wide_store8(uint4* xw, int n_pad, int nblk, int t, int e0, uint4 packed, float sum32) {
+    const int pass = t / n_pad, n = t - pass * n_pad;
+    uint4* blk = xw + (size_t)(pass * nblk + (e0 >> 8)) * WIDE_CHUNKS * n_pad;
+    const int cb = (e0 >> 6) & 3, c = (e0 >> 3) & 7;
+    blk[(size_t)(cb * n_pad + n) * 8 + (c ^ (n & 7))] = packed;
+    if ((e0 & 24) == 0) {
+        const int sub = (e0 >> 5) & 7;
+        const __half hi = __float2half_rn(sum32);
+        reinterpret_cast<__half2*>(blk + (size_t)(32 + (sub >> 2)) * n_pad + n)[sub & 3] = __halves2half2(hi, __float2half_rn(sum32 - __half2float(hi)));
+    }
+}
 // Pack eight f16 values (natural order) into the operand's stored order.
 __device__ __forceinline__ uint4 act_pack8(const __half (&h)[8]) {
     uint4 o;
@@ -171,9 +190,8 @@ __device__ __forceinline__ uint4 act_pack8(const __half (&h)[8]) {
 // Device helper for producers of matmul inputs: a thread that holds eight consecutive f32 outputs v[0..8) of
 // column e0 (a multiple of 8) of token t stores them, rounded to f16, into the operand; the thread holding the
 // even run of each 16-column pair also stores the pair's sum.  Threads of a warp must hold consecutive runs
-// (lane i and lane i^1 form a pair) and all 32 lanes must call it together.
-__device__ __forceinline__ void act_store8(const float (&v)[8], uint4* xp, uint4* xs, int t, int e0, int nblk,
-                                           bool active) {
+// (lane i and lane i^1 form a pair; lanes 4i .. 4i + 3 a 32-column run) and all 32 lanes must call it together.
+__device__ __forceinline__ void act_store8(const float (&v)[8], const ActOut& act, int row, int e0, int nblk, bool active) {
     __half h[8];
     float s = 0.f;
 #pragma unroll
@@ -183,9 +201,15 @@ __device__ __forceinline__ void act_store8(const float (&v)[8], uint4* xp, uint4
     }
     if (!active) s = 0.f;
     s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if (active) {
-        xp[act_xp_index(t, e0, nblk)] = act_pack8(h);
-        if ((e0 & 8) == 0) act_store_sum16(xs, t, e0, nblk, s);
+    const int t = act.row0 + row;
+    if (act.wide == 0) {
+        if (active) {
+            act.xp[act_xp_index(t, e0, nblk)] = act_pack8(h);
+            if ((e0 & 8) == 0) act_store_sum16(act.xs, t, e0, nblk, s);
+        }
+        return;
     }
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (active) wide_store8(act.xp, act.wide, nblk, t, e0, act_pack8(h), s);
 }
 #endif

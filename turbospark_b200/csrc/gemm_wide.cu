@@ -52,7 +52,6 @@ constexpr int WIDE_B_STAGES = 3;     // activation ring: 3 stages up to 64 token
 constexpr int WIDE_NMAX = 128;       // token rows per pass
 constexpr int WIDE_NDUAL = 64;       // up to here two blocks' A operands fit beside the accumulators, and three activation stages
 constexpr int WIDE_NTWO = 96;        // up to here two accumulators of the mins' products fit tensor memory
-constexpr int WIDE_CHUNKS = 34;      // 32 chunks of 8 K positions + 2 chunks of 32-column sums per block
 constexpr int WIDE_A_COLS = 64;      // tensor-memory columns of one A slot: 128 f16 K positions, half a block
 constexpr int WIDE_MIN_BYTES = WM * 16 * 2;  // the mins step's A operand: 128 rows x 16 K positions of f16
 constexpr int WIDE_SCALE_SLOTS = 8;  // a block's scales are written at most four blocks before it is folded
@@ -120,7 +119,7 @@ __global__ void __launch_bounds__(256) wide_prepare_kernel(const __half* __restr
         reinterpret_cast<__half2*>(&tile[32 + (sub >> 2)][w])[sub & 3] = hl;
     }
     __syncthreads();
-    uint4* dst = xw + (size_t)pass * units * WIDE_CHUNKS * per_pass + (size_t)blk * WIDE_CHUNKS * n_pad;
+    uint4* dst = xw + (size_t)(pass * units + blk) * WIDE_CHUNKS * n_pad;
     // eight tokens are one swizzle group: 1024 bytes per 64-column block, then the sums of the whole pass
     for (int i = threadIdx.x; i < 32 * 8; i += 256) {
         const int cb = i >> 6, t = (i >> 3) & 7, c = i & 7;
@@ -539,8 +538,8 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             }
         }
         if (!ok && lane == 0) bars->failed = 1;
+        pdl_launch_dependents();  // by the warps that have waited: who starts then may rely on everything before this launch
     }
-    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == WIDE_WARP_MMA) {
@@ -595,6 +594,12 @@ static bool wide_takes_many(const WidePlan& p, int sm_count, int n_tiles, int un
     const int64_t many = ((int64_t)n_tiles * passes + sm_count - 1) / sm_count * units;
     return many <= passes * one;
 }
+static int wide_pass_rows(int tokens) {
+    const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX;
+    return ((tokens + passes - 1) / passes + 15) / 16 * 16;
+}
+// (rows behind the last token are left as they are: a token row's products do not meet another's)
+ActOut wide_operand(void* workspace, int tokens) { return ActOut{static_cast<uint4*>(workspace), nullptr, wide_pass_rows(tokens), 0}; }
 // the operand copy of every pass of a call with `tokens` token rows
 size_t gemm_wide_workspace_bytes(int64_t cols, int tokens) {
     const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX;
@@ -674,14 +679,15 @@ cudaError_t launch_gemm_wide_q4k(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w
     CUtensorMap wmap;
     if (cudaError_t e = wide_weight_map(w, rows, units, &wmap); e != cudaSuccess) return e;
     // token rows go through in equal passes of at most WIDE_NMAX; one launch lays out the operand of every pass
-    const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX;
-    const int n_pad = ((tokens + passes - 1) / passes + 15) / 16 * 16;
+    const int passes = (tokens + WIDE_NMAX - 1) / WIDE_NMAX, n_pad = wide_pass_rows(tokens);
     const size_t pass_chunks = (size_t)units * WIDE_CHUNKS * n_pad;
     uint4* xw = static_cast<uint4*>(workspace);
     if (!workspace)
         if (cudaError_t e = cudaMallocAsync((void**)&xw, pass_chunks * passes * 16, st); e != cudaSuccess) return e;
-    cudaError_t e = tsb_launch(ctx, wide_prepare_kernel, dim3((unsigned)units, (unsigned)(passes * (n_pad >> 3))), dim3(256), 0, st, true, x,
-                               x_stride, tokens, n_pad, units, xw);
+    cudaError_t e = cudaSuccess;
+    if (x)
+        e = tsb_launch(ctx, wide_prepare_kernel, dim3((unsigned)units, (unsigned)(passes * (n_pad >> 3))), dim3(256), 0, st, true, x, x_stride, tokens, n_pad,
+                       units, xw);
     const WidePlan plan = wide_plan(ctx->sm_count, rows, units);
     const int n_tiles = (int)(rows / WM), ksplit = plan.ksplit;
     const size_t smem = wide_smem_bytes(n_pad);

@@ -15,20 +15,32 @@ namespace {
 // memory (double precision exp/sin/cos rounded once, which reproduces a correctly
 // rounded f32 libm: crates/compute/src/rope.rs:208-255), then every head is
 // rotated with NeoX pairing (i, head_dim/2 + i).
+__device__ __forceinline__ void rope_angle(int i, int hd, float log_theta, int position, float* c, float* s) {
+    const float exponent = -((float)(2 * i)) / (float)hd;
+    const float freq = (float)exp((double)__fmul_rn(exponent, log_theta));
+    const float angle = __fmul_rn((float)position, freq);
+    *c = (float)cos((double)angle), *s = (float)sin((double)angle);
+}
+// The same angles once for a pass of many layers: [rows][head_dim], cos then sin.  (Worked out anew by every layer's launch they
+// were most of its 10.7 us at 65 rows.)
+__global__ void rope_table_kernel(const tsb_row_desc* __restrict__ rows, int hd, float log_theta, float* __restrict__ table) {
+    pdl_wait();
+    const int r = blockIdx.x, half = hd >> 1, position = rows[r].position;
+    float* t = table + (size_t)r * hd;
+    for (int i = threadIdx.x; i < half; i += blockDim.x) rope_angle(i, hd, log_theta, position, &t[i], &t[half + i]);
+    pdl_launch_dependents();
+}
 __global__ void rope_store_kv_kernel(KvView kv, int layer, __half* __restrict__ qkv, const tsb_row_desc* __restrict__ rows,
-                                     int n_q_heads, float log_theta, uint32_t* __restrict__ err) {
+                                     int n_q_heads, float log_theta, const float* __restrict__ table, uint32_t* __restrict__ err) {
     extern __shared__ float cs[];  // cos[half], sin[half]
     pdl_wait();
     const int r = blockIdx.x;
     const tsb_row_desc rd = rows[r];
     const int hd = kv.head_dim, half = hd >> 1;
-    const float pos = (float)rd.position;
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        const float exponent = -((float)(2 * i)) / (float)hd;
-        const float freq = (float)exp((double)__fmul_rn(exponent, log_theta));
-        const float angle = __fmul_rn(pos, freq);
-        cs[i] = (float)cos((double)angle);
-        cs[half + i] = (float)sin((double)angle);
+    if (table) {
+        for (int i = threadIdx.x; i < hd; i += blockDim.x) cs[i] = table[(size_t)r * hd + i];
+    } else {
+        for (int i = threadIdx.x; i < half; i += blockDim.x) rope_angle(i, hd, log_theta, rd.position, &cs[i], &cs[half + i]);
     }
     __syncthreads();
     pdl_launch_dependents();
@@ -40,17 +52,20 @@ __global__ void rope_store_kv_kernel(KvView kv, int layer, __half* __restrict__ 
         if (threadIdx.x == 0) atomicCAS(err, 0u, (uint32_t)TSB_DEV_BAD_INDEX);
         return;
     }
-    // q heads in place, k heads into the cache
-    for (int idx = threadIdx.x; idx < (n_q_heads + nkv) * half; idx += blockDim.x) {
-        const int h = idx / half, i = idx - h * half;
+    // q heads in place, k heads into the cache; eight pairs per thread
+    for (int idx = threadIdx.x; idx < (n_q_heads + nkv) * (half >> 3); idx += blockDim.x) {
+        const int h = idx / (half >> 3), i0 = (idx - h * (half >> 3)) * 8;
         const __half* src = row + (size_t)h * hd;
-        const float x0 = __half2float(src[i]), x1 = __half2float(src[half + i]);
-        const float c = cs[i], s = cs[half + i];
-        const __half o0 = __float2half_rn(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)));
-        const __half o1 = __float2half_rn(__fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)));
+        uint4 lo = *reinterpret_cast<const uint4*>(src + i0), hi = *reinterpret_cast<const uint4*>(src + half + i0);
+        __half *l = reinterpret_cast<__half*>(&lo), *u = reinterpret_cast<__half*>(&hi);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float x0 = __half2float(l[i]), x1 = __half2float(u[i]), c = cs[i0 + i], s = cs[half + i0 + i];
+            l[i] = __float2half_rn(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)));
+            u[i] = __float2half_rn(__fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)));
+        }
         __half* dst = h < n_q_heads ? row + (size_t)h * hd : krow + (size_t)(h - n_q_heads) * hd;
-        dst[i] = o0;
-        dst[half + i] = o1;
+        *reinterpret_cast<uint4*>(dst + i0) = lo, *reinterpret_cast<uint4*>(dst + half + i0) = hi;
     }
     // v heads: straight copy
     const uint4* vsrc = reinterpret_cast<const uint4*>(row + (size_t)(n_q_heads + nkv) * hd);
@@ -257,9 +272,12 @@ int32_t kv_fill_keys(tsb_kv* kv, cudaStream_t st, int32_t seq, int64_t tokens, u
 }
 
 cudaError_t launch_rope_store_kv(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, __half* qkv,
-                                 const tsb_row_desc* rows_dev, int rows, int n_q_heads, float theta) {
+                                 const tsb_row_desc* rows_dev, int rows, int n_q_heads, float theta, const float* table) {
     return tsb_launch(ctx, rope_store_kv_kernel, dim3((unsigned)rows), dim3(256), (size_t)kv->view.head_dim * sizeof(float),
-                      st, true, kv->view, layer, qkv, rows_dev, n_q_heads, logf(theta), ctx->dev_error);
+                      st, true, kv->view, layer, qkv, rows_dev, n_q_heads, logf(theta), table, ctx->dev_error);
+}
+cudaError_t launch_rope_table(tsb_ctx* ctx, cudaStream_t st, const tsb_row_desc* rows_dev, int rows, int head_dim, float theta, float* table) {
+    return tsb_launch(ctx, rope_table_kernel, dim3((unsigned)rows), dim3(64), 0, st, true, rows_dev, head_dim, logf(theta), table);
 }
 
 extern "C" {
@@ -442,7 +460,7 @@ int32_t tsb_rope_store_kv(tsb_ctx* ctx, tsb_stream s, tsb_kv* kv, int32_t layer,
     TSB_REQUIRE(ctx, layer >= 0 && layer < kv->view.layers, "layer %d outside 0..%d", layer, kv->view.layers);
     TSB_REQUIRE(ctx, kv->view.pool, "a plain cache takes no rotated f16 rows");
     DeviceGuard g(ctx);
-    TSB_CUDA(ctx, launch_rope_store_kv(ctx, (cudaStream_t)s, kv, layer, (__half*)qkv_f16, rows_dev, rows, n_q_heads, theta));
+    TSB_CUDA(ctx, launch_rope_store_kv(ctx, (cudaStream_t)s, kv, layer, (__half*)qkv_f16, rows_dev, rows, n_q_heads, theta, nullptr));
     return TSB_OK;
 }
 

@@ -86,7 +86,7 @@ struct ModelRt {
     // largest pass has 24 rows or more) with natural-layout f16 buffers around it; otherwise every pass runs the
     // register path.  Never a mix: the two sum in different orders.
     bool wide_ok = false;
-    __half *w_xn = nullptr, *w_qkv = nullptr, *w_ao = nullptr, *w_o = nullptr, *w_gu = nullptr, *w_a = nullptr, *w_logits = nullptr;
+    __half *w_xn = nullptr, *w_qkv = nullptr, *w_o = nullptr, *w_gu = nullptr, *w_logits = nullptr;
     void* w_ws = nullptr;
     void* w_part = nullptr;  // split sums of the matmuls with few row tiles
     // routed feed-forward: router logits [R, E] f32, picks [R, k], weights [R, k] f16, a zero residual, workspace

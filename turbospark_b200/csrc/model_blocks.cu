@@ -478,7 +478,7 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
     const int W = std::max(R, rt.prompt_rows);  // rows of the buffers a prompt's pass uses
     if ((rc = A((size_t)W * c.d_model * 2, (void**)&rt.h))) return rc;
     if ((rc = A((size_t)R * c.n_q_heads * c.head_dim * 2, (void**)&rt.q))) return rc;
-    if ((rc = A((size_t)R * c.head_dim * sizeof(float), (void**)&rt.cs))) return rc;
+    if ((rc = A((size_t)W * c.head_dim * sizeof(float), (void**)&rt.cs))) return rc;
     if ((rc = A((size_t)(2 * c.n_layers + 1) * R * (c.d_model / 16) * sizeof(float), (void**)&rt.ss))) return rc;
     const int64_t od = (int64_t)c.n_q_heads * c.head_dim;
     if ((rc = A(act_xp_bytes(Rp, c.d_model), (void**)&rt.act_d.xp)) || (rc = A(act_xs_bytes(Rp, c.d_model), (void**)&rt.act_d.xs))) return rc;
@@ -516,9 +516,8 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
     }
     if (wide) {
         const int64_t widest = std::max<int64_t>(std::max<int64_t>(c.d_model, od), c.ffn);
-        if ((rc = A((size_t)W * c.d_model * 2, (void**)&rt.w_xn)) || (rc = A((size_t)W * qkv_dim * 2, (void**)&rt.w_qkv)) ||
-            (rc = A((size_t)W * od * 2, (void**)&rt.w_ao)) || (rc = A((size_t)W * c.d_model * 2, (void**)&rt.w_o)) ||
-            (rc = A((size_t)W * 2 * c.ffn * 2, (void**)&rt.w_gu)) || (rc = A((size_t)W * c.ffn * 2, (void**)&rt.w_a)) ||
+        if ((rc = A((size_t)W * qkv_dim * 2, (void**)&rt.w_qkv)) || (rc = A((size_t)W * c.d_model * 2, (void**)&rt.w_o)) ||
+            (rc = A((size_t)W * 2 * c.ffn * 2, (void**)&rt.w_gu)) ||
             (rc = A((size_t)R * c.vocab * 2, (void**)&rt.w_logits)) || (rc = A(gemm_wide_workspace_bytes(widest, W), &rt.w_ws)))
             return rc;
         size_t part = gemm_wide_partial_bytes(ctx, model->lm_head.rows, model->lm_head.cols);
@@ -542,24 +541,27 @@ static cudaError_t forward_device_wide(tsb_session* s, ModelRt& rt, const int32_
     const tsb_model* m = rt.model;
     const tsb_model_config& c = m->cfg;
     const float scale = 1.0f / sqrtf((float)c.head_dim);
+    // every matmul's operand is written in place by the kernel before it: norm, attention merge, activation
+    const ActOut next = wide_operand(rt.w_ws, rows);
     // A prompt's groups attend like streams of one pass - a group sees the ones before it as committed rows, which the launch before
     // has just written - as many at a time as their shares fit the scratch; the last, shorter one on its own.
-    auto attend_prompt = [&](int L, int64_t od, int64_t qkv_dim) -> cudaError_t {
+    auto attend_prompt = [&](int L, int64_t qkv_dim) -> cudaError_t {
         for (int r0 = 0; r0 < rows;) {
             const int per = std::min(PROMPT_GROUP, rows - r0);
             int groups = (rows - r0) / per;
             auto shares = [&](int g) { return (int64_t)g * per * attn_prompt_splits(max_len); };
             const int64_t room = (int64_t)(rt.attn_scratch_bytes / ((size_t)c.n_q_heads * (c.head_dim + 2) * sizeof(float)));
             while (groups > 1 && shares(groups) > room) groups = (groups + 1) / 2;
-            cudaError_t e = launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv + r0 * qkv_dim, qkv_dim, rt.w_ao + r0 * od, ActOut{nullptr, nullptr}, rows_dev + r0,
+            ActOut group = next;
+            group.row0 = r0;
+            cudaError_t e = launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv + r0 * qkv_dim, qkv_dim, nullptr, group, rows_dev + r0,
                                                     groups * per, per, c.n_q_heads, scale, max_len, rt.attn_scratch, rt.attn_rows, true);
             if (e != cudaSuccess) return e;
             r0 += groups * per;
         }
         return cudaSuccess;
     };
-    const int64_t od = (int64_t)c.n_q_heads * c.head_dim, qkv_dim = (int64_t)(c.n_q_heads + 2 * c.n_kv_heads) * c.head_dim;
-    const ActOut none{nullptr, nullptr};
+    const int64_t qkv_dim = (int64_t)(c.n_q_heads + 2 * c.n_kv_heads) * c.head_dim;
     cudaError_t e;
 #define FW(x)                           \
     do {                                \
@@ -567,34 +569,35 @@ static cudaError_t forward_device_wide(tsb_session* s, ModelRt& rt, const int32_
         if (e != cudaSuccess) return e; \
     } while (0)
     FW(launch_embed_rows(ctx, st, m->embed.qtype, m->embed.data, c.vocab, c.d_model, tokens_dev, token_stride, rows, rt.h, 1.0f));
-    FW(launch_rmsnorm_rows(ctx, st, rt.h, nullptr, m->layers[0].attn_norm, rt.w_xn, none, rows, c.d_model, c.rms_eps));
+    FW(launch_rope_table(ctx, st, rows_dev, rows, c.head_dim, c.rope_theta, rt.cs));
+    FW(launch_rmsnorm_rows(ctx, st, rt.h, nullptr, m->layers[0].attn_norm, nullptr, next, rows, c.d_model, c.rms_eps));
     for (int L = 0; L < c.n_layers; L++) {
         const LayerW& l = m->layers[L];
-        FW(launch_gemm_wide_q4k(ctx, st, l.wqkv.data, l.wqkv.rows, l.wqkv.cols, rt.w_xn, c.d_model, rows, rt.w_qkv, qkv_dim, false, rt.w_ws, rt.w_part));
-        FW(launch_rope_store_kv(ctx, st, rt.kv, L, rt.w_qkv, rows_dev, rows, c.n_q_heads, c.rope_theta));
+        FW(launch_gemm_wide_q4k(ctx, st, l.wqkv.data, l.wqkv.rows, l.wqkv.cols, nullptr, 0, rows, rt.w_qkv, qkv_dim, false, rt.w_ws, rt.w_part));
+        FW(launch_rope_store_kv(ctx, st, rt.kv, L, rt.w_qkv, rows_dev, rows, c.n_q_heads, c.rope_theta, rt.cs));
         if (prompt)
-            FW(attend_prompt(L, od, qkv_dim));
+            FW(attend_prompt(L, qkv_dim));
         else
-            FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv, qkv_dim, rt.w_ao, none, rows_dev, rows, rows_per_seq, c.n_q_heads, scale,
+            FW(launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv, qkv_dim, nullptr, next, rows_dev, rows, rows_per_seq, c.n_q_heads, scale,
                                        max_len, rt.attn_scratch, rt.attn_rows));
-        FW(launch_gemm_wide_q4k(ctx, st, l.wo.data, l.wo.rows, l.wo.cols, rt.w_ao, od, rows, rt.w_o, c.d_model, false, rt.w_ws, rt.w_part));
-        FW(launch_rmsnorm_rows(ctx, st, rt.h, rt.w_o, l.ffn_norm, rt.w_xn, none, rows, c.d_model, c.rms_eps));
-        FW(launch_gemm_wide_q4k(ctx, st, l.wgu.data, l.wgu.rows, l.wgu.cols, rt.w_xn, c.d_model, rows, rt.w_gu, 2 * (int64_t)c.ffn, false, rt.w_ws, rt.w_part));
-        FW(launch_silu_mul(ctx, st, rt.w_gu, rt.w_gu + c.ffn, rt.w_a, none, rows, c.ffn, 2 * (int64_t)c.ffn, c.ffn));
-        FW(launch_gemm_wide_q4k(ctx, st, l.wdown.data, l.wdown.rows, l.wdown.cols, rt.w_a, c.ffn, rows, rt.w_o, c.d_model, false, rt.w_ws, rt.w_part));
+        FW(launch_gemm_wide_q4k(ctx, st, l.wo.data, l.wo.rows, l.wo.cols, nullptr, 0, rows, rt.w_o, c.d_model, false, rt.w_ws, rt.w_part));
+        FW(launch_rmsnorm_rows(ctx, st, rt.h, rt.w_o, l.ffn_norm, nullptr, next, rows, c.d_model, c.rms_eps));
+        FW(launch_gemm_wide_q4k(ctx, st, l.wgu.data, l.wgu.rows, l.wgu.cols, nullptr, 0, rows, rt.w_gu, 2 * (int64_t)c.ffn, false, rt.w_ws, rt.w_part));
+        FW(launch_silu_mul(ctx, st, rt.w_gu, rt.w_gu + c.ffn, nullptr, next, rows, c.ffn, 2 * (int64_t)c.ffn, c.ffn));
+        FW(launch_gemm_wide_q4k(ctx, st, l.wdown.data, l.wdown.rows, l.wdown.cols, nullptr, 0, rows, rt.w_o, c.d_model, false, rt.w_ws, rt.w_part));
         const void* g = L + 1 < c.n_layers ? (const void*)m->layers[L + 1].attn_norm : (const void*)m->out_norm;
-        FW(launch_rmsnorm_rows(ctx, st, rt.h, rt.w_o, g, rt.w_xn, none, rows, c.d_model, c.rms_eps));
+        FW(launch_rmsnorm_rows(ctx, st, rt.h, rt.w_o, g, nullptr, next, rows, c.d_model, c.rms_eps));
     }
     if (logits) {
         if (last_rows_only && rows_per_seq > 1) {
             // every row's logits into the staging buffer, then each stream's last row to its place
-            FW(launch_gemm_wide_q4k(ctx, st, m->lm_head.data, m->lm_head.rows, m->lm_head.cols, rt.w_xn, c.d_model, rows, rt.w_logits, c.vocab,
+            FW(launch_gemm_wide_q4k(ctx, st, m->lm_head.data, m->lm_head.rows, m->lm_head.cols, nullptr, 0, rows, rt.w_logits, c.vocab,
                                     false, rt.w_ws, rt.w_part));
             FW(cudaMemcpy2DAsync(logits, (size_t)logits_stride * 2, rt.w_logits + (size_t)(rows_per_seq - 1) * c.vocab,
                                  (size_t)rows_per_seq * c.vocab * 2, (size_t)c.vocab * 2, (size_t)(rows / rows_per_seq),
                                  cudaMemcpyDeviceToDevice, st));
         } else {
-            FW(launch_gemm_wide_q4k(ctx, st, m->lm_head.data, m->lm_head.rows, m->lm_head.cols, rt.w_xn, c.d_model, rows, logits, logits_stride,
+            FW(launch_gemm_wide_q4k(ctx, st, m->lm_head.data, m->lm_head.rows, m->lm_head.cols, nullptr, 0, rows, logits, logits_stride,
                                     false, rt.w_ws, rt.w_part));
         }
     }

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 #pragma unroll
                 for (int i = 0; i < 8; i++) o[i] = 0.f;
             }
-            act_store8(o, act.xp, act.xs, r, active ? e0 : 0, d >> 8, active);
+            act_store8(o, act, r, active ? e0 : 0, d >> 8, active);
         }
     }
 }
@@ -264,7 +264,7 @@ __global__ void silu_mul_kernel(const __half* __restrict__ gate, const __half* _
         for (int i = 0; i < 8; i++) pp[i] = __float2half_rn(o[i]);
         *reinterpret_cast<uint4*>(out + (size_t)r * out_stride + e0) = pk;
     }
-    if (act.xp) act_store8(o, act.xp, act.xs, r, e0, n >> 8, active);
+    if (act.xp) act_store8(o, act, r, e0, n >> 8, active);
 }
 
 __global__ void residual_add_kernel(__half* __restrict__ x, const __half* __restrict__ y, int64_t n) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256)
             }
             *reinterpret_cast<uint4*>(h + (size_t)r * d + e0) = hv;
         }
-        act_store8(xg, act.xp, act.xs, r, active ? e0 : 0, d >> 8, active);
+        act_store8(xg, act, r, active ? e0 : 0, d >> 8, active);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
