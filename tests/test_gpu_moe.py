@@ -150,3 +150,11 @@ def test_a_model_with_a_routed_feed_forward_matches_the_oracle_forward(oracle):
     spec_hist, spec_emit, res = sess.spec_run(prompt, rc)
     assert np.array_equal(seq_emit, spec_emit) and res.new_tokens == 24
     sess.close(), draft.close(), target.close(), ctx.close()
+
+
+@pytest.mark.parametrize("kind,tokens,experts,k,d,f", [(2, 40, 8, 4, 512, 256), (2, 70, 4, 2, 768, 512), (1, 20, 8, 2, 512, 256), (0, 33, 8, 4, 1024, 1024),
+                                                        (2, 64, 32, 8, 1024, 768), (4, 12, 8, 2, 256, 256)])
+def test_narrow_down_projections_match_the_oracle(ctx, oracle, kind, tokens, experts, k, d, f):
+    """Down projections of one to four blocks a row take several row tiles per stage: every number of blocks, counts of tiles that
+    leave a remainder, every token-tile width."""
+    test_routed_feed_forward_matches_the_oracle(ctx, oracle, kind, tokens, experts, k, d, f)
