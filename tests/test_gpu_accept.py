@@ -354,3 +354,47 @@ def test_rows_counted_by_value_match_the_oracle(ctx, oracle, vocab, batch, kind)
             assert outs[b].status == 0 and outs[b].accepted == acc and outs[b].draws == draws, (shape, b)
             assert list(outs[b].tokens[:acc + 1]) == list(toks), (shape, b, list(outs[b].tokens[:acc + 1]), list(toks))
     assert checked > 0
+
+
+@pytest.mark.parametrize("temperature", [1e-310, 3e-3, 20.0, 1e4])
+def test_temperatures_at_the_ends_of_their_range_match_the_oracle(ctx, oracle, temperature):
+    """Below 5.6e-309 the reciprocal of a temperature overflows; at high ones entries whose exponential or its quotient by the sum is
+    subnormal, or zero, keep the weight that the quotient leaves them: 30000 entries share the maximum, the others lie 700 to 748 below,
+    around where the exponential (745.1) and its quotient by such a sum (745.1 - ln 30000 = 734.8) vanish."""
+    import turbospark_b200 as tsb
+    rng = np.random.default_rng(17)
+    batch, k, vocab = 24, 1, 60001
+    tgt = (370.0 - np.round(rng.uniform(700.0, 748.0, (batch, k + 1, vocab)) * 4) / 4).astype(np.float32)
+    for b in range(batch):
+        for r in range(k + 1):
+            tgt[b, r, rng.permutation(vocab)[:30000]] = 370.0
+    drf = np.roll(tgt[:, :k], 1, axis=2)
+    t16, d16 = oracle.f32_to_f16_bits(tgt), oracle.f32_to_f16_bits(drf)
+    ocfg = oracle.shaping(temperature=temperature, seed=4)
+    props = rng.integers(0, vocab, size=(batch, k)).astype(np.int32)
+    unis = (np.linspace(0.02, 0.998, batch * (2 * k + 1)) * 2.0**64).astype(np.uint64)
+    unis = rng.permutation(unis).reshape(batch, 2 * k + 1)
+    outs = _run_accept(ctx, oracle, t16, d16, props, unis, temperature)
+    # the f32 rows of the history path: a penalty that meets no token of a history of one unlikely entry
+    cfg = tsb.shaping(temperature=temperature, seed=4, presence_penalty=0.25)
+    ocfg_h = oracle.shaping(temperature=temperature, seed=4, presence_penalty=0.25)
+    hist = [np.array([7], dtype=np.int32)] * batch
+    outs_h = _run_accept_history(ctx, t16, d16, props, unis, cfg, hist, [0] * batch)
+    checked = 0
+    for b in range(batch):
+        for got, want in ((outs[b], oracle.accept_round(t16[b], d16[b], props[b], ocfg, unis[b])),
+                          (outs_h[b], oracle.accept_round(t16[b], d16[b], props[b], ocfg_h, unis[b], hist[b], 0))):
+            acc, toks, draws, margins = want
+            if margins[0] < 1e-13 or margins[1] < 1e-11:  # decided within rounding: two entries of one value are the rule here
+                continue
+            checked += 1
+            assert got.status == 0 and got.accepted == acc and list(got.tokens[:acc + 1]) == list(toks), (b, got.accepted, acc, list(got.tokens[:2]), toks)
+    assert checked >= batch
+    rows, uni = t16[:, 0].copy(), unis[:, 0].copy()
+    toks, margins = ctx.alloc(batch * 4), ctx.alloc(batch * 8)
+    ctx.sample(ctx.to_device(rows), ctx.to_device(uni), batch, vocab, tsb.shaping(temperature=temperature, seed=4), toks, margins,
+               ctx.alloc(ctx.accept_scratch_bytes(batch, 0, vocab)))
+    ctx.sync()
+    for b, got in enumerate(toks.download(np.int32, batch)):
+        want, margin = oracle.sample(rows[b], ocfg, int(uni[b]))
+        assert margin < 1e-11 or got == want, (b, got, want)

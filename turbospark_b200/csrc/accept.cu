@@ -105,11 +105,20 @@ __device__ unsigned long long* g_sample_trace = nullptr;  // development builds:
 // w_i of reweight (choose.rs:296-321): ((e_i / sum) / top)^(1/T) with top = max_i e_i / sum = 1 / sum and e_i = exp(x),
 // x = logit - max, which is exp(x / T): one exponential of an exactly known argument instead of an exponential, two
 // divisions and a power, which were most of the time of an acceptance.
-// An e that underflows to zero keeps the weight zero at every temperature.
-__device__ __forceinline__ double weight_of(double x, double inv_t, bool unit_t) {
-    if (unit_t) return exp(x);
-    return x < -745.13321910194122 ? 0.0 : exp(x * inv_t);
+// Far below the maximum the two part: e and e / sum become subnormal and then zero, a weight that no high temperature brings back.
+// There - a sum of up to 163840 exponentials keeps e / sum normal down to x = -696 - the quotients are taken as they stand.
+// (Rare, so the power is a call: inlined, its registers would be every entry's.)
+constexpr double QUOTIENTS_BELOW = -690.0;
+__device__ __noinline__ double weight_of_quotients(double x, double inv_t, double sum) {
+    const double p = exp(x) / sum, top = 1.0 / sum;
+    return p > 0.0 ? pow(p / top, inv_t) : 0.0;
 }
+__device__ __forceinline__ double weight_of(double x, double inv_t, bool unit_t, double sum) {
+    if (unit_t) return exp(x);
+    return x >= QUOTIENTS_BELOW ? exp(x * inv_t) : weight_of_quotients(x, inv_t, sum);
+}
+// 1 / T.  Where that overflows, the largest finite number: 0 * inv_t of the top entry stays 0, every other entry's weight is 0.
+__device__ __forceinline__ double inverse_temperature(double t) { return fmin(1.0 / t, 1.7976931348623157e308); }
 
 __device__ __forceinline__ double block_sum_f64(double v, double* red) {
     // fixed shape: lane tree, then warps in index order
@@ -417,7 +426,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
             s += e;
         }
         const double sum = cluster_sum_f64(cluster, &xch, 0, block_sum_f64(s, red));
-        const double inv_t = 1.0 / temperature;
+        const double inv_t = inverse_temperature(temperature);
         const bool unit_t = temperature == 1.0;
         st.sum = sum;
         const bool truncating = (tr.top_k > 0 && tr.top_k < (unsigned)vocab) || tr.top_p > 0.0 || tr.min_p > 0.0;
@@ -425,7 +434,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
         double t = 0.0;
         for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS)
             if (!truncating || survives_e(st, row[sl.lo + j], sl.lo + j, ecache[j]))
-                t += unit_t ? ecache[j] : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t);
+                t += unit_t ? ecache[j] : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
         st.total = cluster_sum_f64(cluster, &xch, 1, block_sum_f64(t, red));
     }
     pdl_launch_dependents();
@@ -692,7 +701,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
         for (int i = 0; i < KEY_SETS_MAX / 2; i++)
             if (2 * i < sets) reinterpret_cast<uint2*>(hist)[i * ACC_THREADS + threadIdx.x] = make_uint2(sums[2 * i], sums[2 * i + 1]);
         __syncthreads();
-        const double dmx = (double)st.max, inv_t = 1.0 / temperature;
+        const double dmx = (double)st.max, inv_t = inverse_temperature(temperature);
         const bool unit_t = temperature == 1.0;
         double s = 0.0;
         for (int i = threadIdx.x; i < keys; i += ACC_THREADS)
@@ -729,7 +738,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
                 if (!n) continue;
                 const double x = (double)value_of_key16(key) - dmx;
                 if (st.min_e > 0.0 && (x < log_min || !(exp(x) >= st.min_e))) continue;
-                t += (double)n * weight_of(x, inv_t, unit_t);
+                t += (double)n * weight_of(x, inv_t, unit_t, sum);
             }
             t = cluster_sum_f64(cluster, &c.xch, 1, block_sum_f64(t, c.red));
         }
@@ -745,7 +754,7 @@ template <typename LT>
 __device__ __forceinline__ double prob_of(const LT* row, const RowStats& st, int token, double inv_t, bool unit_t) {
     const double x = (double)Logit<LT>::val(row[token]) - (double)st.max;
     if (!survives(st, row[token], token, x)) return 0.0;  // distribution.rs:61-66: not in the support
-    return st.total > 0.0 ? weight_of(x, inv_t, unit_t) / st.total : 0.0;
+    return st.total > 0.0 ? weight_of(x, inv_t, unit_t, st.sum) / st.total : 0.0;
 }
 
 // What is drawn from: (a) the shaped row prow, or (b) the residual max(p - q, 0) of two shaped rows.
@@ -762,10 +771,10 @@ struct Mass {
         const double x = (double)Logit<LT>::val(lp) - (double)ps->max;
         *in_support = survives(*ps, lp, idx, x);
         if (!*in_support) return 0.0;
-        double m = weight_of(x, inv_t, unit_t) * p_inv;
+        double m = weight_of(x, inv_t, unit_t, ps->sum) * p_inv;
         if (qrow) {
             const double xq = (double)Logit<LT>::val(lq) - (double)qs->max;
-            if (survives(*qs, lq, idx, xq)) m = fmax(m - weight_of(xq, inv_t, unit_t) * q_inv, 0.0);
+            if (survives(*qs, lq, idx, xq)) m = fmax(m - weight_of(xq, inv_t, unit_t, qs->sum) * q_inv, 0.0);
             *in_support = m > 0.0;
         }
         return m;
@@ -869,7 +878,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
     const int32_t* prop = proposals + (size_t)b * prop_stride;
     const uint64_t* un = uniforms + (size_t)b * rps;
     const bool sampled = temperature != 0.0;
-    const double inv_t = sampled ? 1.0 / temperature : 1.0;
+    const double inv_t = sampled ? inverse_temperature(temperature) : 1.0;
     const bool unit_t = temperature == 1.0;
     const Slice sl = my_slice(vocab, rank);
 
@@ -1018,7 +1027,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
     } else if (temperature == 0.0) {
         token = am;
     } else {
-        const double dmx = (double)mx, inv_t = 1.0 / temperature;
+        const double dmx = (double)mx, inv_t = inverse_temperature(temperature);
         const bool unit_t = temperature == 1.0;
         const bool truncating = (tr.top_k > 0 && tr.top_k < (unsigned)vocab) || tr.top_p > 0.0 || tr.min_p > 0.0;
         // e = exp(l - max) and its sum (and, when every entry survives, the last entry in rank order on the way)
@@ -1053,7 +1062,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
             // At temperature 1 the reference's weight ((e/sum)/top with top = 1/sum) is e up to two roundings.  The
             // few-ulp difference can move a draw only when the target lies within ~1e-15 of a boundary, which the
             // reported margin shows.
-            const double w = unit_t ? e : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t);
+            const double w = unit_t ? e : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
             ecache[j] = w;
             acc += w;
             const unsigned long long eb = (unsigned long long)__double_as_longlong(e);
