@@ -398,3 +398,21 @@ def test_temperatures_at_the_ends_of_their_range_match_the_oracle(ctx, oracle, t
     for b, got in enumerate(toks.download(np.int32, batch)):
         want, margin = oracle.sample(rows[b], ocfg, int(uni[b]))
         assert margin < 1e-11 or got == want, (b, got, want)
+
+
+@pytest.mark.parametrize("shape", [dict(temperature=1.0), dict(temperature=0.7), dict(temperature=0.8, top_p=0.9), dict(temperature=1.2, top_k=50, min_p=0.01)])
+def test_a_streams_record_does_not_depend_on_its_batch(ctx, oracle, shape):
+    """Alone, among eight and among eighty streams a row gets clusters of eight, four and two; margins and tokens stay bit for bit."""
+    rng = np.random.default_rng(23)
+    batch, k, vocab = 80, 2, 20011
+    t16, d16 = _logits(oracle, rng, batch, k, vocab)
+    props = np.argmax(oracle.f16_bits_to_f32(d16), axis=2).astype(np.int32)
+    unis = rng.integers(0, 2**63, size=(batch, 2 * k + 1)).astype(np.uint64) * np.uint64(2)
+    record = lambda o: (o.status, o.accepted, o.draws, list(o.tokens), o.margin_accept, o.margin_draw)  # noqa: E731
+    want = [record(o) for o in _run_accept(ctx, oracle, t16, d16, props, unis, **shape)]
+    for b in range(0, batch, 8):
+        some = [record(o) for o in _run_accept(ctx, oracle, t16[b:b + 8], d16[b:b + 8], props[b:b + 8], unis[b:b + 8], **shape)]
+        assert some == want[b:b + 8], b
+    for b in range(8):
+        alone = _run_accept(ctx, oracle, t16[b:b + 1], d16[b:b + 1], props[b:b + 1], unis[b:b + 1], **shape)
+        assert record(alone[0]) == want[b], b

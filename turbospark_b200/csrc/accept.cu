@@ -456,8 +456,13 @@ __global__ void __launch_bounds__(ACC_THREADS)
 //
 // After the count, CTA r of n owns the keys [r, r + 1) * 65536 / n in key order (descending value): it adds the members'
 // 16-bit counters of its keys and keeps the sums as 32-bit words in the place of its own counters.
+//
+// Sums of f64 run over blocks of 8192 keys, each summed in the same shape and added in key order, so that a row's record does
+// not depend on how many CTAs it got - that is, on how many streams its acceptance has.
 constexpr int KEYS = 65536;
 constexpr int KEY_SETS_MAX = KEYS / 2 / ACC_THREADS;  // keys a thread owns in a cluster of two
+constexpr int KEY_BLOCK = KEYS / CL;
+constexpr int KEY_BLOCKS_MAX = KEYS / 2 / KEY_BLOCK;  // blocks of a CTA in a cluster of two
 
 __device__ __forceinline__ float value_of_key16(uint32_t key) {
     return __half2float(__ushort_as_half((unsigned short)((key & 0x8000u) ? key : (key ^ 0x7FFFu))));
@@ -470,7 +475,8 @@ __device__ __forceinline__ uint32_t key16_of_bits(uint32_t u) {
 struct KeyShared {
     unsigned long long group[KEY_SETS_MAX * 32];  // mass of each run of 32 keys, in key order
     unsigned long long scan[ACC_THREADS / 32];
-    double red[ACC_THREADS / 32];
+    double red[KEY_BLOCKS_MAX][ACC_THREADS / 32];
+    double part[2][KEY_BLOCKS_MAX];  // a CTA's block sums, for its peers: of the exponentials, of the weights
     Xchg xch;
     uint32_t best[ACC_THREADS / 32];
     uint32_t sel_group;
@@ -488,6 +494,31 @@ __device__ __forceinline__ unsigned long long warp_scan_u64(unsigned long long v
         if ((threadIdx.x & 31) >= o) v += n;
     }
     return v;
+}
+
+// The sum of term(key) over the cluster's occupied keys (see above); slot: which exchange area.  Same in every CTA.
+template <class TermFn>
+__device__ double cluster_sum_keys(cg::cluster_group& cluster, KeyShared& c, int slot, int keys, TermFn term) {
+    const int blocks = keys / KEY_BLOCK, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int b = 0; b < blocks; b++) {
+        double t = 0.0;
+        for (int i = b * KEY_BLOCK + threadIdx.x; i < (b + 1) * KEY_BLOCK; i += ACC_THREADS) t += term(i);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) c.red[b][warp] = t;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < blocks) {
+        double t = 0.0;
+        for (int w = 0; w < ACC_THREADS / 32; w++) t += c.red[threadIdx.x][w];
+        c.part[slot][threadIdx.x] = t;
+    }
+    cluster.sync();
+    double t = 0.0;
+    const int n = (int)cluster.num_blocks();
+    for (int r = 0; r < n; r++)
+        for (int b = 0; b < blocks; b++) t += cluster.map_shared_rank(&c, r)->part[slot][b];
+    return t;
 }
 
 // Entry number `target` (0-based, in units of mass) of the row in rank order: which key, the how-manieth entry of that
@@ -703,10 +734,10 @@ __global__ void __launch_bounds__(ACC_THREADS)
         __syncthreads();
         const double dmx = (double)st.max, inv_t = inverse_temperature(temperature);
         const bool unit_t = temperature == 1.0;
-        double s = 0.0;
-        for (int i = threadIdx.x; i < keys; i += ACC_THREADS)
-            if (const uint32_t n = hist[i]) s += (double)n * exp((double)value_of_key16(key0 + i) - dmx);
-        const double sum = cluster_sum_f64(cluster, &c.xch, 0, block_sum_f64(s, c.red));
+        const double sum = cluster_sum_keys(cluster, c, 0, keys, [&](int i) {
+            const uint32_t n = hist[i];
+            return n ? (double)n * exp((double)value_of_key16(key0 + i) - dmx) : 0.0;
+        });
         st.sum = sum;
         // ---- the cut: the first top_k entries, cut further where the cumulative e / sum first reaches top_p
         st.min_e = tr.min_p > 0.0 ? tr.min_p : 0.0;
@@ -729,18 +760,16 @@ __global__ void __launch_bounds__(ACC_THREADS)
         if (st.has_cut && cut_occ + 1 < cut_count) st.cut_idx = cluster_find_entry(cluster, c, row, sl, st.cut_key, cut_occ);
         double t = sum;
         if (st.has_cut || st.min_e > 0.0 || !unit_t) {
-            t = 0.0;
             const double log_min = st.min_e > 0.0 ? log(st.min_e) - 1e-9 : 0.0;  // surely below the floor: no exp needed
-            for (int i = threadIdx.x; i < keys; i += ACC_THREADS) {
+            t = cluster_sum_keys(cluster, c, 1, keys, [&](int i) {
                 uint32_t n = hist[i];
                 const uint32_t key = key0 + i;
                 if (st.has_cut && key >= st.cut_key) n = key == st.cut_key ? (uint32_t)cut_occ + 1 : 0;
-                if (!n) continue;
+                if (!n) return 0.0;
                 const double x = (double)value_of_key16(key) - dmx;
-                if (st.min_e > 0.0 && (x < log_min || !(exp(x) >= st.min_e))) continue;
-                t += (double)n * weight_of(x, inv_t, unit_t, sum);
-            }
-            t = cluster_sum_f64(cluster, &c.xch, 1, block_sum_f64(t, c.red));
+                if (st.min_e > 0.0 && (x < log_min || !(exp(x) >= st.min_e))) return 0.0;
+                return (double)n * weight_of(x, inv_t, unit_t, sum);
+            });
         }
         st.total = t;
     }
