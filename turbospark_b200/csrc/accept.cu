@@ -106,16 +106,19 @@ __device__ unsigned long long* g_sample_trace = nullptr;  // development builds:
 // x = logit - max, which is exp(x / T): one exponential of an exactly known argument instead of an exponential, two
 // divisions and a power, which were most of the time of an acceptance.
 // Far below the maximum the two part: e and e / sum become subnormal and then zero, a weight that no high temperature brings back.
-// There - a sum of up to 163840 exponentials keeps e / sum normal down to x = -696 - the quotients are taken as they stand.
-// (Rare, so the power is a call: inlined, its registers would be every entry's.)
-constexpr double QUOTIENTS_BELOW = -690.0;
+// There - a sum of up to 163840 exponentials keeps e / sum normal down to x = -696 - the quotients are taken as they stand.  Up to
+// a temperature of ten such weights are below 1e-29: nothing to a total of at least 1, to a mass in units of 2^-60 or to a decision whose
+// margin is not itself below 1e-29.  So only the kernels for higher temperatures (HOT) have the power compiled in; its registers are every entry's.
+constexpr double QUOTIENTS_BELOW = -690.0, HOT_ABOVE = 10.0;
 __device__ __noinline__ double weight_of_quotients(double x, double inv_t, double sum) {
     const double p = exp(x) / sum, top = 1.0 / sum;
     return p > 0.0 ? pow(p / top, inv_t) : 0.0;
 }
+template <bool HOT>
 __device__ __forceinline__ double weight_of(double x, double inv_t, bool unit_t, double sum) {
     if (unit_t) return exp(x);
-    return x >= QUOTIENTS_BELOW ? exp(x * inv_t) : weight_of_quotients(x, inv_t, sum);
+    if (x >= QUOTIENTS_BELOW) return exp(x * inv_t);
+    return HOT ? weight_of_quotients(x, inv_t, sum) : 0.0;
 }
 // 1 / T.  Where that overflows, the largest finite number: 0 * inv_t of the top entry stays 0, every other entry's weight is 0.
 __device__ __forceinline__ double inverse_temperature(double t) { return fmin(1.0 / t, 1.7976931348623157e308); }
@@ -357,7 +360,7 @@ __device__ void cluster_find_cut(cg::cluster_group& cluster, DrawShared& c, cons
 
 // ---------------------------------------------------------------- statistics
 // One cluster per row: max / first argmax / finiteness, sum_i exp(l_i - max), total = sum_i w_i.
-template <typename LT>
+template <typename LT, bool HOT>
 __global__ void __launch_bounds__(ACC_THREADS)
     accept_stats_kernel(const LT* __restrict__ target, const LT* __restrict__ draft, int k, int vocab,
                         double temperature, TruncShape tr, RowStats* __restrict__ stats, int rows_per_stream) {
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
         double t = 0.0;
         for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS)
             if (!truncating || survives_e(st, row[sl.lo + j], sl.lo + j, ecache[j]))
-                t += unit_t ? ecache[j] : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
+                t += unit_t ? ecache[j] : weight_of<HOT>((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
         st.total = cluster_sum_f64(cluster, &xch, 1, block_sum_f64(t, red));
     }
     pdl_launch_dependents();
@@ -452,13 +455,15 @@ __global__ void __launch_bounds__(ACC_THREADS)
 // at most 65535 entries: a cluster of 2 CTAs holds vocabularies up to 131068, of 4 or 8 the rest.  More CTAs per row
 // shorten a row while SMs are idle; see stats_half_ctas for the rule.
 // Measured, acceptance of 32 streams x 5 proposals, 128256 entries, temperature 0.8, top-p 0.95 (352 rows): this kernel 286 us where
-// the entry-by-entry one took 1700; at temperature 1 without truncation, both launches, 64 streams: 415 us (1240 before), one: 67 (107).
+// the entry-by-entry one took 1700; both launches, temperature 0.8 without truncation, one stream and 32: 8192 entries 44 and 162 us (46
+// and 347 before), 128256 entries 71 and 282 (151 and 1185).  The fixed cost shows below 1024 entries alone: 512 and one stream 40 us
+// (36 before), 32 streams 142 (299).
 //
 // After the count, CTA r of n owns the keys [r, r + 1) * 65536 / n in key order (descending value): it adds the members'
 // 16-bit counters of its keys and keeps the sums as 32-bit words in the place of its own counters.
 //
-// Sums of f64 run over blocks of 8192 keys, each summed in the same shape and added in key order, so that a row's record does
-// not depend on how many CTAs it got - that is, on how many streams its acceptance has.
+// Sums of f64 have one order whatever the cluster's size (cluster_sum_keys), so that a row's record does not depend on how many
+// CTAs it got - that is, on how many streams its acceptance has.
 constexpr int KEYS = 65536;
 constexpr int KEY_SETS_MAX = KEYS / 2 / ACC_THREADS;  // keys a thread owns in a cluster of two
 constexpr int KEY_BLOCK = KEYS / CL;
@@ -473,9 +478,12 @@ __device__ __forceinline__ uint32_t key16_of_bits(uint32_t u) {
 }
 
 struct KeyShared {
-    unsigned long long group[KEY_SETS_MAX * 32];  // mass of each run of 32 keys, in key order
+    union {  // (the two together would take the L1's share that the search for an entry reads its row through)
+        unsigned long long group[KEY_SETS_MAX * 32];  // a search: mass of each run of 32 keys, in key order
+        double column[KEY_BLOCKS_MAX][ACC_THREADS];   // a sum: see cluster_sum_keys
+    };
     unsigned long long scan[ACC_THREADS / 32];
-    double red[KEY_BLOCKS_MAX][ACC_THREADS / 32];
+    double red[ACC_THREADS / 32];
     double part[2][KEY_BLOCKS_MAX];  // a CTA's block sums, for its peers: of the exponentials, of the weights
     Xchg xch;
     uint32_t best[ACC_THREADS / 32];
@@ -496,28 +504,40 @@ __device__ __forceinline__ unsigned long long warp_scan_u64(unsigned long long v
     return v;
 }
 
-// The sum of term(key) over the cluster's occupied keys (see above); slot: which exchange area.  Same in every CTA.
-template <class TermFn>
-__device__ double cluster_sum_keys(cg::cluster_group& cluster, KeyShared& c, int slot, int keys, TermFn term) {
-    const int blocks = keys / KEY_BLOCK, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// The sum over the cluster's keys: add(i, t) adds key i's term to t; slot: which exchange area.  Same in every CTA, and the same
+// whatever the cluster's size: a block of 8192 keys is 1024 columns (key mod 1024) of eight keys, the columns meet in a fixed tree and the
+// blocks are added in key order.  The first levels of the tree go through shared memory: 64-bit shuffles of every block's sums cost more
+// than the sums.
+template <class AddFn>
+__device__ double cluster_sum_keys(cg::cluster_group& cluster, KeyShared& c, int slot, int keys, AddFn add) {
+    const int blocks = keys / KEY_BLOCK, lane = threadIdx.x & 31;
     for (int b = 0; b < blocks; b++) {
         double t = 0.0;
-        for (int i = b * KEY_BLOCK + threadIdx.x; i < (b + 1) * KEY_BLOCK; i += ACC_THREADS) t += term(i);
+#pragma unroll
+        for (int i = 0; i < KEY_BLOCK; i += ACC_THREADS) add(b * KEY_BLOCK + i + threadIdx.x, t);
+        c.column[b][threadIdx.x] = t;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < blocks * 256) {
+        const double* col = c.column[threadIdx.x >> 8] + (threadIdx.x & 255);
+        double t = (col[0] + col[256]) + (col[512] + col[768]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) c.red[b][warp] = t;
+        if (lane == 0) c.red[threadIdx.x >> 5] = t;
     }
     __syncthreads();
     if ((int)threadIdx.x < blocks) {
         double t = 0.0;
-        for (int w = 0; w < ACC_THREADS / 32; w++) t += c.red[threadIdx.x][w];
+#pragma unroll
+        for (int w = 0; w < 8; w++) t += c.red[threadIdx.x * 8 + w];
         c.part[slot][threadIdx.x] = t;
     }
     cluster.sync();
+    // one load per warp, a block per lane, instead of a chain of remote loads
+    const double v = lane < CL ? cluster.map_shared_rank(&c, lane / blocks)->part[slot][lane % blocks] : 0.0;
     double t = 0.0;
-    const int n = (int)cluster.num_blocks();
-    for (int r = 0; r < n; r++)
-        for (int b = 0; b < blocks; b++) t += cluster.map_shared_rank(&c, r)->part[slot][b];
+#pragma unroll
+    for (int b = 0; b < CL; b++) t += __shfl_sync(0xffffffffu, v, b);
     return t;
 }
 
@@ -631,6 +651,7 @@ __device__ int cluster_find_entry(cg::cluster_group& cluster, KeyShared& c, cons
     return root->found_idx;
 }
 
+template <bool HOT>
 __global__ void __launch_bounds__(ACC_THREADS)
     accept_stats_half_kernel(const __half* __restrict__ target, const __half* __restrict__ draft, int k, int vocab, double temperature,
                              TruncShape tr, RowStats* __restrict__ stats, int rows_per_stream) {
@@ -734,9 +755,8 @@ __global__ void __launch_bounds__(ACC_THREADS)
         __syncthreads();
         const double dmx = (double)st.max, inv_t = inverse_temperature(temperature);
         const bool unit_t = temperature == 1.0;
-        const double sum = cluster_sum_keys(cluster, c, 0, keys, [&](int i) {
-            const uint32_t n = hist[i];
-            return n ? (double)n * exp((double)value_of_key16(key0 + i) - dmx) : 0.0;
+        const double sum = cluster_sum_keys(cluster, c, 0, keys, [&](int i, double& s) {
+            if (const uint32_t n = hist[i]) s += (double)n * exp((double)value_of_key16(key0 + i) - dmx);
         });
         st.sum = sum;
         // ---- the cut: the first top_k entries, cut further where the cumulative e / sum first reaches top_p
@@ -761,14 +781,14 @@ __global__ void __launch_bounds__(ACC_THREADS)
         double t = sum;
         if (st.has_cut || st.min_e > 0.0 || !unit_t) {
             const double log_min = st.min_e > 0.0 ? log(st.min_e) - 1e-9 : 0.0;  // surely below the floor: no exp needed
-            t = cluster_sum_keys(cluster, c, 1, keys, [&](int i) {
+            t = cluster_sum_keys(cluster, c, 1, keys, [&](int i, double& s) {
                 uint32_t n = hist[i];
                 const uint32_t key = key0 + i;
                 if (st.has_cut && key >= st.cut_key) n = key == st.cut_key ? (uint32_t)cut_occ + 1 : 0;
-                if (!n) return 0.0;
+                if (!n) return;
                 const double x = (double)value_of_key16(key) - dmx;
-                if (st.min_e > 0.0 && (x < log_min || !(exp(x) >= st.min_e))) return 0.0;
-                return (double)n * weight_of(x, inv_t, unit_t, sum);
+                if (st.min_e > 0.0 && (x < log_min || !(exp(x) >= st.min_e))) return;
+                s += (double)n * weight_of<HOT>(x, inv_t, unit_t, sum);
             });
         }
         st.total = t;
@@ -779,15 +799,15 @@ __global__ void __launch_bounds__(ACC_THREADS)
 }
 
 // probability of one token under a row's shaped distribution (distribution.rs:61-66 over the full support)
-template <typename LT>
+template <typename LT, bool HOT>
 __device__ __forceinline__ double prob_of(const LT* row, const RowStats& st, int token, double inv_t, bool unit_t) {
     const double x = (double)Logit<LT>::val(row[token]) - (double)st.max;
     if (!survives(st, row[token], token, x)) return 0.0;  // distribution.rs:61-66: not in the support
-    return st.total > 0.0 ? weight_of(x, inv_t, unit_t, st.sum) / st.total : 0.0;
+    return st.total > 0.0 ? weight_of<HOT>(x, inv_t, unit_t, st.sum) / st.total : 0.0;
 }
 
 // What is drawn from: (a) the shaped row prow, or (b) the residual max(p - q, 0) of two shaped rows.
-template <typename LT>
+template <typename LT, bool HOT>
 struct Mass {
     const LT* prow;
     const LT* qrow;  // null: (a)
@@ -800,10 +820,10 @@ struct Mass {
         const double x = (double)Logit<LT>::val(lp) - (double)ps->max;
         *in_support = survives(*ps, lp, idx, x);
         if (!*in_support) return 0.0;
-        double m = weight_of(x, inv_t, unit_t, ps->sum) * p_inv;
+        double m = weight_of<HOT>(x, inv_t, unit_t, ps->sum) * p_inv;
         if (qrow) {
             const double xq = (double)Logit<LT>::val(lq) - (double)qs->max;
-            if (survives(*qs, lq, idx, xq)) m = fmax(m - weight_of(xq, inv_t, unit_t, qs->sum) * q_inv, 0.0);
+            if (survives(*qs, lq, idx, xq)) m = fmax(m - weight_of<HOT>(xq, inv_t, unit_t, qs->sum) * q_inv, 0.0);
             *in_support = m > 0.0;
         }
         return m;
@@ -812,8 +832,8 @@ struct Mass {
 
 // Fills fp[] (this CTA's slice) with the fixed-point probability of every token.  Returns false when the residual is
 // empty or below the reference's 1e-12 floor.
-template <typename LT>
-__device__ bool cluster_fill_masses(cg::cluster_group& cluster, DrawShared& c, unsigned long long* fp, const Mass<LT>& mass, Slice sl) {
+template <typename LT, bool HOT>
+__device__ bool cluster_fill_masses(cg::cluster_group& cluster, DrawShared& c, unsigned long long* fp, const Mass<LT, HOT>& mass, Slice sl) {
     double* raw = reinterpret_cast<double*>(fp);  // the same storage holds f64 masses first, fixed point after
     double t = 0.0;
     int any = 0;
@@ -857,8 +877,8 @@ __device__ bool cluster_fill_masses(cg::cluster_group& cluster, DrawShared& c, u
 
 // The last support entry in rank order - smallest exp, then the largest index - which a target past the last cumulative
 // sum (rounding of the masses) draws.  Rare, so the search runs only then; every CTA of the cluster takes part.
-template <typename LT>
-__device__ int cluster_last_support(cg::cluster_group& cluster, DrawShared& c, const Mass<LT>& mass, Slice sl) {
+template <typename LT, bool HOT>
+__device__ int cluster_last_support(cg::cluster_group& cluster, DrawShared& c, const Mass<LT, HOT>& mass, Slice sl) {
     unsigned long long best = ~0ull;
     unsigned int best_i = 0;
     for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS) {
@@ -884,7 +904,7 @@ __device__ int cluster_last_support(cg::cluster_group& cluster, DrawShared& c, c
 
 __device__ __forceinline__ double unit_interval(uint64_t v) { return (double)(v >> 11) * (1.0 / 9007199254740992.0); }
 
-template <typename LT>
+template <typename LT, bool HOT>
 __global__ void __launch_bounds__(ACC_THREADS)
     accept_decide_kernel(const LT* __restrict__ target, const LT* __restrict__ draft,
                          const int32_t* __restrict__ proposals, int prop_stride, const uint64_t* __restrict__ uniforms,
@@ -916,7 +936,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
     if (sampled && (int)threadIdx.x < 2 * k) {
         const int i = threadIdx.x >> 1, side = threadIdx.x & 1, x = prop[i];
         const RowStats& rs = st[side ? k + 1 + i : i];
-        s_prob[side][i] = x >= 0 && x < vocab && !rs.nonfinite ? prob_of((side ? drows : trows) + (size_t)i * vocab, rs, x, inv_t, unit_t) : 0.0;
+        s_prob[side][i] = x >= 0 && x < vocab && !rs.nonfinite ? prob_of<LT, HOT>((side ? drows : trows) + (size_t)i * vocab, rs, x, inv_t, unit_t) : 0.0;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -959,16 +979,16 @@ __global__ void __launch_bounds__(ACC_THREADS)
         } else {
             const uint64_t u = un[s_draws];
             const unsigned long long tgt = (unsigned long long)(u >> 11) << 7;  // k * 2^-53 in 2^-60 units
-            Mass<LT> mass{prow, nullptr, &st[accepted], nullptr, inv_t, 1.0 / st[accepted].total, 0.0, unit_t};
+            Mass<LT, HOT> mass{prow, nullptr, &st[accepted], nullptr, inv_t, 1.0 / st[accepted].total, 0.0, unit_t};
             bool have = false;
             if (s_rejected) {
                 mass.qrow = drows + (size_t)accepted * vocab, mass.qs = &st[k + 1 + accepted], mass.q_inv = 1.0 / mass.qs->total;
-                have = cluster_fill_masses<LT>(cluster, c, fp, mass, sl);
+                have = cluster_fill_masses<LT, HOT>(cluster, c, fp, mass, sl);
                 if (!have) mass.qrow = nullptr;
             }
-            if (!have) cluster_fill_masses<LT>(cluster, c, fp, mass, sl);
+            if (!have) cluster_fill_masses<LT, HOT>(cluster, c, fp, mass, sl);
             token = cluster_radix_draw<LT>(cluster, c, fp, prow, sl, tgt, &gap);
-            if (token < 0) token = cluster_last_support<LT>(cluster, c, mass, sl), gap = 0;
+            if (token < 0) token = cluster_last_support<LT, HOT>(cluster, c, mass, sl), gap = 0;
         }
     }
     pdl_launch_dependents();
@@ -989,7 +1009,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
 
 // Draft-side draw: one cluster per stream, one row each; statistics and draw in one kernel, so exp(l - max) is
 // evaluated once per entry and stays in shared memory (first as e, then as the weight, then as the fixed-point mass).
-template <typename LT>
+template <typename LT, bool HOT>
 __global__ void __launch_bounds__(ACC_THREADS)
     sample_kernel(const LT* __restrict__ logits, int64_t logits_stride, const uint64_t* __restrict__ uniforms,
                   int uni_stride, int vocab, double temperature, TruncShape tr, int32_t* __restrict__ tokens, int token_stride,
@@ -1091,7 +1111,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
             // At temperature 1 the reference's weight ((e/sum)/top with top = 1/sum) is e up to two roundings.  The
             // few-ulp difference can move a draw only when the target lies within ~1e-15 of a boundary, which the
             // reported margin shows.
-            const double w = unit_t ? e : weight_of((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
+            const double w = unit_t ? e : weight_of<HOT>((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
             ecache[j] = w;
             acc += w;
             const unsigned long long eb = (unsigned long long)__double_as_longlong(e);
@@ -1193,16 +1213,16 @@ int32_t check_shaping(tsb_ctx* ctx, const tsb_shaping* sh, bool have_history = f
 size_t slice_smem(int vocab) { return (size_t)(((vocab + CL - 1) / CL + 1) & ~1) * sizeof(unsigned long long); }
 
 // the cluster kernels keep a vocabulary slice in dynamic shared memory (opt-in per device, per instantiation)
-template <typename LT>
+template <typename LT, bool HOT>
 cudaError_t configure_kernels(const tsb_ctx* ctx) {
     static SmemOptIn stats_done, decide_done, sample_done;
     cudaError_t e = cudaSuccess;
     if constexpr (sizeof(LT) == 2)
-        e = tsb_opt_in_smem(ctx, accept_stats_half_kernel, (size_t)KEYS * 2, stats_done);
+        e = tsb_opt_in_smem(ctx, accept_stats_half_kernel<HOT>, (size_t)KEYS * 2, stats_done);
     else
-        e = tsb_opt_in_smem(ctx, accept_stats_kernel<LT>, (size_t)SLICE_MAX * 8, stats_done);
-    if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, accept_decide_kernel<LT>, (size_t)SLICE_MAX * 8, decide_done);
-    if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, sample_kernel<LT>, (size_t)SLICE_MAX * 8, sample_done);
+        e = tsb_opt_in_smem(ctx, accept_stats_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, stats_done);
+    if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, accept_decide_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, decide_done);
+    if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, sample_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, sample_done);
     return e;
 }
 
@@ -1290,34 +1310,41 @@ static int stats_half_ctas(int sm_count, int rows, int vocab) {
     return n;
 }
 
-template <typename LT>
+template <typename LT, bool HOT>
 static cudaError_t launch_stats(tsb_ctx* ctx, cudaStream_t st, const LT* target, const LT* draft, int rows, int k, int vocab, double temperature,
                                 TruncShape tr, RowStats* stats, int rows_per_stream) {
     if constexpr (sizeof(LT) == 2) {
         const int n = stats_half_ctas(ctx->sm_count, rows, vocab);
-        return tsb_launch_cluster(ctx, accept_stats_half_kernel, dim3((unsigned)(rows * n)), dim3(ACC_THREADS), (size_t)KEYS * 2, st, true, (unsigned)n, target,
+        return tsb_launch_cluster(ctx, accept_stats_half_kernel<HOT>, dim3((unsigned)(rows * n)), dim3(ACC_THREADS), (size_t)KEYS * 2, st, true, (unsigned)n, target,
                                   draft, k, vocab, temperature, tr, stats, rows_per_stream);
     } else {
-        return tsb_launch_cluster(ctx, accept_stats_kernel<LT>, dim3((unsigned)(rows * CL)), dim3(ACC_THREADS), slice_smem(vocab), st, true, (unsigned)CL, target,
-                                  draft, k, vocab, temperature, tr, stats, rows_per_stream);
+        return tsb_launch_cluster(ctx, accept_stats_kernel<LT, HOT>, dim3((unsigned)(rows * CL)), dim3(ACC_THREADS), slice_smem(vocab), st, true, (unsigned)CL,
+                                  target, draft, k, vocab, temperature, tr, stats, rows_per_stream);
     }
 }
 
+template <typename LT, bool HOT>
+static cudaError_t launch_accept_th(tsb_ctx* ctx, cudaStream_t st, const LT* target, const LT* draft, const int32_t* proposals,
+                                    int prop_stride, const uint64_t* uniforms, int batch, int k, int vocab, AcceptShape shape,
+                                    tsb_accept_out* out_dev, int32_t* next_tokens, int next_stride, void* scratch) {
+    RowStats* stats = reinterpret_cast<RowStats*>(scratch);
+    const int rps = 2 * k + 1;
+    const size_t smem = slice_smem(vocab);
+    if (cudaError_t e = configure_kernels<LT, HOT>(ctx); e != cudaSuccess) return e;
+    const TruncShape tr{shape.top_k, shape.top_p, shape.min_p};
+    const double temperature = shape.temperature;
+    cudaError_t e = launch_stats<LT, HOT>(ctx, st, target, draft, batch * rps, k, vocab, temperature, tr, stats, rps);
+    if (e != cudaSuccess) return e;
+    return tsb_launch_cluster(ctx, accept_decide_kernel<LT, HOT>, dim3((unsigned)(batch * CL)), dim3(ACC_THREADS), smem, st, true,
+                              (unsigned)CL, target, draft, proposals, prop_stride, uniforms, k, vocab, temperature,
+                              (const RowStats*)stats, out_dev, next_tokens, next_stride);
+}
 template <typename LT>
 static cudaError_t launch_accept_t(tsb_ctx* ctx, cudaStream_t st, const LT* target, const LT* draft, const int32_t* proposals,
                                    int prop_stride, const uint64_t* uniforms, int batch, int k, int vocab, AcceptShape shape,
                                    tsb_accept_out* out_dev, int32_t* next_tokens, int next_stride, void* scratch) {
-    RowStats* stats = reinterpret_cast<RowStats*>(scratch);
-    const int rps = 2 * k + 1;
-    const size_t smem = slice_smem(vocab);
-    if (cudaError_t e = configure_kernels<LT>(ctx); e != cudaSuccess) return e;
-    const TruncShape tr{shape.top_k, shape.top_p, shape.min_p};
-    const double temperature = shape.temperature;
-    cudaError_t e = launch_stats<LT>(ctx, st, target, draft, batch * rps, k, vocab, temperature, tr, stats, rps);
-    if (e != cudaSuccess) return e;
-    return tsb_launch_cluster(ctx, accept_decide_kernel<LT>, dim3((unsigned)(batch * CL)), dim3(ACC_THREADS), smem, st, true,
-                              (unsigned)CL, target, draft, proposals, prop_stride, uniforms, k, vocab, temperature,
-                              (const RowStats*)stats, out_dev, next_tokens, next_stride);
+    auto launch = shape.temperature > HOT_ABOVE ? launch_accept_th<LT, true> : launch_accept_th<LT, false>;
+    return launch(ctx, st, target, draft, proposals, prop_stride, uniforms, batch, k, vocab, shape, out_dev, next_tokens, next_stride, scratch);
 }
 
 cudaError_t launch_accept(tsb_ctx* ctx, cudaStream_t st, LogitRows target, LogitRows draft, const int32_t* proposals,
@@ -1330,17 +1357,24 @@ cudaError_t launch_accept(tsb_ctx* ctx, cudaStream_t st, LogitRows target, Logit
                                    out_dev, next_tokens, next_stride, scratch);
 }
 
+template <typename LT, bool HOT>
+static cudaError_t launch_sample_th(tsb_ctx* ctx, cudaStream_t st, const LT* logits, int64_t logits_stride, const uint64_t* uniforms,
+                                    int uni_stride, int batch, int vocab, AcceptShape shape, int32_t* tokens_dev, int token_stride,
+                                    double* margins_dev) {
+    const TruncShape tr{shape.top_k, shape.top_p, shape.min_p};
+    const double temperature = shape.temperature;
+    const size_t smem = slice_smem(vocab);
+    if (cudaError_t e = configure_kernels<LT, HOT>(ctx); e != cudaSuccess) return e;
+    return tsb_launch_cluster(ctx, sample_kernel<LT, HOT>, dim3((unsigned)(batch * CL)), dim3(ACC_THREADS), smem, st, true, (unsigned)CL,
+                              logits, logits_stride, uniforms, uni_stride, vocab, temperature, tr, tokens_dev, token_stride,
+                              margins_dev, ctx->dev_error);
+}
 template <typename LT>
 static cudaError_t launch_sample_t(tsb_ctx* ctx, cudaStream_t st, const LT* logits, int64_t logits_stride, const uint64_t* uniforms,
                                    int uni_stride, int batch, int vocab, AcceptShape shape, int32_t* tokens_dev, int token_stride,
                                    double* margins_dev) {
-    const TruncShape tr{shape.top_k, shape.top_p, shape.min_p};
-    const double temperature = shape.temperature;
-    const size_t smem = slice_smem(vocab);
-    if (cudaError_t e = configure_kernels<LT>(ctx); e != cudaSuccess) return e;
-    return tsb_launch_cluster(ctx, sample_kernel<LT>, dim3((unsigned)(batch * CL)), dim3(ACC_THREADS), smem, st, true, (unsigned)CL,
-                              logits, logits_stride, uniforms, uni_stride, vocab, temperature, tr, tokens_dev, token_stride,
-                              margins_dev, ctx->dev_error);
+    auto launch = shape.temperature > HOT_ABOVE ? launch_sample_th<LT, true> : launch_sample_th<LT, false>;
+    return launch(ctx, st, logits, logits_stride, uniforms, uni_stride, batch, vocab, shape, tokens_dev, token_stride, margins_dev);
 }
 
 cudaError_t launch_sample(tsb_ctx* ctx, cudaStream_t st, LogitRows logits, int64_t logits_stride,
@@ -1435,11 +1469,11 @@ cudaError_t launch_argmax_rows(tsb_ctx* ctx, cudaStream_t st, LogitRows logits, 
     RowStats* stats = reinterpret_cast<RowStats*>(scratch);
     const TruncShape none{0u, 0.0, 0.0};
     if (logits.f32) {
-        if (cudaError_t e = configure_kernels<float>(ctx); e != cudaSuccess) return e;
-        return launch_stats<float>(ctx, st, (const float*)logits.p, nullptr, n_rows, n_rows - 1, vocab, 0.0, none, stats, n_rows);
+        if (cudaError_t e = configure_kernels<float, false>(ctx); e != cudaSuccess) return e;
+        return launch_stats<float, false>(ctx, st, (const float*)logits.p, nullptr, n_rows, n_rows - 1, vocab, 0.0, none, stats, n_rows);
     }
-    if (cudaError_t e = configure_kernels<__half>(ctx); e != cudaSuccess) return e;
-    return launch_stats<__half>(ctx, st, (const __half*)logits.p, nullptr, n_rows, n_rows - 1, vocab, 0.0, none, stats, n_rows);
+    if (cudaError_t e = configure_kernels<__half, false>(ctx); e != cudaSuccess) return e;
+    return launch_stats<__half, false>(ctx, st, (const __half*)logits.p, nullptr, n_rows, n_rows - 1, vocab, 0.0, none, stats, n_rows);
 }
 
 int accept_row_stats_bytes() { return (int)sizeof(RowStats); }
