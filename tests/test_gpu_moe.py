@@ -153,8 +153,9 @@ def test_a_model_with_a_routed_feed_forward_matches_the_oracle_forward(oracle):
 
 
 @pytest.mark.parametrize("kind,tokens,experts,k,d,f", [(2, 40, 8, 4, 512, 256), (2, 70, 4, 2, 768, 512), (1, 20, 8, 2, 512, 256), (0, 33, 8, 4, 1024, 1024),
-                                                        (2, 64, 32, 8, 1024, 768), (4, 12, 8, 2, 256, 256)])
+                                                        (2, 64, 32, 8, 1024, 768), (4, 12, 8, 2, 256, 256),
+                                                        (2, 1, 8, 2, 1024, 256), (2, 2, 32, 4, 2048, 256), (0, 6, 16, 4, 2048, 512), (2, 24, 64, 8, 2048, 256)])
 def test_narrow_down_projections_match_the_oracle(ctx, oracle, kind, tokens, experts, k, d, f):
     """Down projections of one to four blocks a row take several row tiles per stage: every number of blocks, counts of tiles that
-    leave a remainder, every token-tile width."""
+    leave a remainder, every token-tile width; few experts with rows, which take fewer tiles per stage than fit, down to one."""
     test_routed_feed_forward_matches_the_oracle(ctx, oracle, kind, tokens, experts, k, d, f)

@@ -116,11 +116,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
     // the same row range's neighbours too - `pack` row tiles side by side, a tile's rows `region` bytes behind its
     // neighbour's - and `units` warps take each.  (The down projections of 128 MXFP4 experts, 2048 x 768, three units: one tile a
     // stage kept five warps idle and paid a stage's hand-shake, barrier and store for 6.5 KB of weights: the routed feed-forward of
-    // 40 rows takes 187 us where it took 203.)
+    // 40 rows takes 184 us where it took 202; 64 rows over 1024 x 256, one unit, 76 where it took 95.)
+    // How many: an item costs its tiles plus about one tile's time, and the items go to the CTAs in waves, so the cheapest number of
+    // tiles is small where few experts have rows.  (Always as many as fit, two experts of 64 tiles and one unit were 20 items of seven
+    // tiles for 296 CTAs: that feed-forward took 15.7 us where one tile a stage takes 12.6; by this rule 12.9.)
     constexpr bool CAN_PACK = GROUPED && EPI == EPI_PLAIN;
     const int region = (units * UB + 30) & ~15;
-    const int pack = CAN_PACK && 2 * units <= STAGE_UNITS ? min(STAGE_UNITS / units, ROW_STRIDE / region) : 1;
-    const int n_groups = CAN_PACK ? (n_tiles + pack - 1) / pack : num_groups<EPI>(n_tiles, epi);
+    const int most = CAN_PACK && 2 * units <= STAGE_UNITS ? min(STAGE_UNITS / units, ROW_STRIDE / region) : 1;
     const int iters = (units + STAGE_UNITS - 1) / STAGE_UNITS;  // stages per row tile
     const int64_t row_bytes = (int64_t)units * UB;
 
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
     // GROUPED: the matrices that take part in this launch, compacted once per CTA (index, row count, first tile), so
     // the item walk touches no global memory and the items spread evenly over the CTAs
     __shared__ int grp_mat[GROUPED ? GROUPED_MAX_MATS : 1], grp_cnt[GROUPED ? GROUPED_MAX_MATS : 1], grp_tile[GROUPED ? GROUPED_MAX_MATS : 1];
-    __shared__ int grp_active;
+    __shared__ int grp_active, grp_pack;
     if constexpr (GROUPED) {
         if (warp == 0) {
             int base = 0;
@@ -150,9 +152,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
                 base += __popc(mask);
             }
             if (lane == 0) grp_active = base;
+            if constexpr (CAN_PACK) {  // lane l: the cost of l + 1 tiles
+                const int waves = (base * ((n_tiles + lane) / (lane + 1)) + (int)gridDim.x - 1) / (int)gridDim.x;
+                const uint32_t cost = lane < most ? (uint32_t)waves * (uint32_t)(lane + 2) : 0x7FFFFFFu;
+                const uint32_t best = __reduce_min_sync(0xffffffffu, min(cost, 0x7FFFFFFu) << 5 | (uint32_t)lane);
+                if (lane == 0) grp_pack = (int)(best & 31u) + 1;
+            }
         }
     }
     __syncthreads();
+    int pack = 1;
+    if constexpr (CAN_PACK) pack = grp_pack;
+    const int n_groups = CAN_PACK ? (n_tiles + pack - 1) / pack : num_groups<EPI>(n_tiles, epi);
     const int n_items = GROUPED ? n_groups * grp_active : n_groups;
 
     // The CTA is persistent: it walks groups blockIdx.x, +gridDim.x, ... and the stage ring runs on across
