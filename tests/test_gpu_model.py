@@ -779,3 +779,55 @@ def test_prompts_in_one_pass_match_the_oracle_and_the_same_prompt_in_portions(ri
     sess.sequential_run(prompt[:n], tsb.run_config(tsb.shaping(temperature=0.0), 1, 1, reuse_prefix=True))
     _close(oracle, sess.produce(int(prompt[n]), n), want, rel=4e-3, abs_=4e-3)
     sess.close()
+
+
+@pytest.fixture(scope="module", params=[(8, 2, 128), (4, 4, 128), (8, 2, 64)], ids=["4 heads of 128", "1 head of 128", "4 heads of 64"])
+def long_rig(oracle, request):
+    """Two layers with a window of several attention cuts: query heads, key heads, head size."""
+    import turbospark_b200 as tsb
+    nq, nkv, hd = request.param
+    ctx = tsb.Ctx(0)
+    cfg = tsb.ModelConfig(2, 512, nq, nkv, hd, 512, 1024, 12288, 1e-6, 1e4)
+    mats, norms = weights.random_weights(cfg, 5, oracle)
+    target = tsb.Model(ctx, cfg)
+    weights.load_weights(target, mats, norms)
+    ot = oracle.Model(oracle.ModelCfg(cfg.n_layers, cfg.d_model, nq, nkv, hd, cfg.ffn, cfg.vocab, cfg.max_context, cfg.rms_eps, cfg.rope_theta), threads=8)
+    weights.load_weights(ot, mats, norms)
+    yield dict(ctx=ctx, cfg=cfg, target=target, ot=ot, tsb=tsb, once=tsb.run_config(tsb.shaping(temperature=0.0), 1, 1))
+    target.close(), ctx.close()
+
+
+@pytest.mark.parametrize("n", [2, 66, 81, 82, 1001, 1026, 1042, 2066, 3001, 9100])
+def test_prompts_of_several_passes_and_cuts_match_the_few_row_path(long_rig, oracle, n):
+    """Prompts whose rows (n - 1) end in groups of 1, 16, 17 and 64 rows, in one pass and several, over one attention cut of 1024
+    positions and several; at 9100 a pass's shares exceed the scratch and its groups go some at a time.  The reference is the
+    session of few rows, which takes a prompt eight rows at a time through other matmul and attention kernels, up to 1042 the oracle too."""
+    tsb, once = long_rig["tsb"], long_rig["once"]
+    prompt = np.random.default_rng(n).integers(0, long_rig["cfg"].vocab, size=n + 1).astype(np.int32)
+    logits = []
+    for max_rows in (32, 8):
+        sess = tsb.Session(long_rig["ctx"], long_rig["target"], None, 1, max_rows)
+        sess.sequential_run(prompt[:n], once)
+        logits.append(sess.produce(int(prompt[n]), n).copy())
+        sess.close()
+    _close(oracle, logits[0], logits[1], rel=4e-3, abs_=4e-3)
+    if n <= 1042:
+        _close(oracle, logits[0], oracle.State(long_rig["ot"]).forward(prompt, 0)[n], rel=4e-3, abs_=4e-3)
+
+
+@pytest.mark.parametrize("short,long", [(3, 66), (11, 300), (74, 128), (82, 1100), (1026, 1600), (1500, 5000), (8300, 9200)])
+def test_a_prompts_rows_do_not_depend_on_the_rows_behind_them(long_rig, short, long):
+    """The cached rows of a prompt are bit for bit those that a longer prompt with the same beginning leaves: whatever the length of
+    their group, their pass, and the number of cuts of the context behind them."""
+    tsb, once = long_rig["tsb"], long_rig["once"]
+    tokens = np.random.default_rng(long).integers(0, long_rig["cfg"].vocab, size=long + 1).astype(np.int32)
+    at = short - 1  # the last token of the shorter one goes through on its own
+    sess = tsb.Session(long_rig["ctx"], long_rig["target"], None, 1, 32)
+    got = []
+    for n in (short, long):
+        sess.reset()
+        sess.sequential_run(tokens[:n], once)
+        sess.rollback_retaining(at, 0)
+        got.append(sess.produce(int(tokens[at]), at).copy())
+    sess.close()
+    assert np.array_equal(got[0], got[1])

@@ -781,22 +781,23 @@ static cudaError_t launch_attn_merge(tsb_ctx* ctx, cudaStream_t st, const float*
 
 cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                     __half* out, ActOut act, const tsb_row_desc* rows_dev, int rows, int rows_per_seq,
-                                    int n_q_heads, float scale, int max_len, void* scratch, int rows_cap, bool prompt) {
+                                    int n_q_heads, float scale, int max_len, void* scratch, int rows_cap, int prompt_chunk) {
+    const bool prompt = prompt_chunk > 0;
     if (attn_split_merge_mode()) {
         // every chunk CTA leaves its share in memory and a second, wide launch merges them (one CTA per row and head)
         const float* part_o;
         const float2* part_ml;
         int n_splits;
-        if (attn_tc_applicable(ctx, kv, rows, rows_per_seq, n_q_heads)) {
+        if (attn_tc_applicable(ctx, kv, rows, rows_per_seq, n_q_heads, prompt)) {
             // many queries per (stream, kv head), or streams enough to fill the device: the tensor-memory kernel; its shares
             // always go through the merge
             cudaError_t e = launch_attn_tc_partials(ctx, st, kv, layer, q, q_stride, rows_dev, rows, rows_per_seq, n_q_heads, scale, max_len,
-                                                    scratch, &part_o, &part_ml, &n_splits, prompt);
+                                                    scratch, &part_o, &part_ml, &n_splits, prompt_chunk);
             if (e != cudaSuccess) return e;
             return launch_attn_merge(ctx, st, part_o, part_ml, n_splits, rows, n_q_heads, kv->view.head_dim, out, act);
         }
         cudaError_t e = launch_attn_partials(ctx, st, kv, layer, q, q_stride, rows_dev, rows, rows_per_seq, n_q_heads, scale, max_len, scratch,
-                                             &part_o, &part_ml, &n_splits, out, act, prompt);
+                                             &part_o, &part_ml, &n_splits, out, act, prompt_chunk);
         if (e != cudaSuccess || n_splits == 1) return e;  // a single split wrote the output itself
         return launch_attn_merge(ctx, st, part_o, part_ml, n_splits, rows, n_q_heads, kv->view.head_dim, out, act);
     }
@@ -830,7 +831,7 @@ cudaError_t launch_attn_decode_rows(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, i
 // CTA every K/V byte of a chunk is in flight from the first instruction.  Like attn_plan it is made for the length rounded up
 // to 512 and does not depend on the row count while the queries fit one tile, so a row gets the same chunks - and
 // the same sums - whether it is verified in a batch or decoded alone.
-static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, bool prompt) {
+static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, int prompt_chunk) {
     AttnPlan p;
     const int G = n_q_heads / kv->view.kv_heads;
     const int n_queries = rows_per_seq * G;
@@ -840,8 +841,8 @@ static AttnPlan attn_plan_partials(const tsb_ctx* ctx, const tsb_kv* kv, int row
     p.n_qtiles = (n_queries + 16 * p.mt - 1) / (16 * p.mt);
     p.groups = rows / rows_per_seq;
     p.cluster_size = 1;
-    if (prompt) {
-        p.chunk = attn_prompt_chunk(max_len), p.n_splits = attn_prompt_splits(max_len);
+    if (prompt_chunk > 0) {
+        p.chunk = prompt_chunk, p.n_splits = attn_prompt_splits(max_len, prompt_chunk);
         return p;
     }
     const int planned = max_len > 0 ? (max_len + 511) / 512 * 512 : 512;
@@ -879,8 +880,8 @@ extern "C" __attribute__((visibility("default"))) void tsb_debug_set_attn_trace(
 cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                  const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int n_q_heads, float scale, int max_len,
                                  void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, __half* out_single,
-                                 ActOut act_single, bool prompt) {
-    const AttnPlan p = attn_plan_partials(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt);
+                                 ActOut act_single, int prompt_chunk) {
+    const AttnPlan p = attn_plan_partials(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt_chunk);
     const int hd = kv->view.head_dim;
     float* part_o = reinterpret_cast<float*>(scratch);
     float2* part_ml = reinterpret_cast<float2*>(part_o + (size_t)rows * n_q_heads * p.n_splits * hd);
@@ -897,7 +898,7 @@ cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int 
     const int defer = single ? 0 : 1;
 #define TSB_ATTN_LAUNCH(HDV, MTV)                                                                                                          \
     return launch_attn_t<HDV, MTV>(ctx, st, p, grid, smem, kv->view, layer, q, q_stride, rows_dev, rows_per_seq, n_q_heads, scale_log2e, part_o, \
-                                   part_ml, ATTN_TICKETS, out, act, defer, prompt)
+                                   part_ml, ATTN_TICKETS, out, act, defer, prompt_chunk > 0)
     if (hd == 128) {
         if (p.mt == 4) TSB_ATTN_LAUNCH(128, 4);
         if (p.mt == 2) TSB_ATTN_LAUNCH(128, 2);
@@ -909,7 +910,7 @@ cudaError_t launch_attn_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int 
 #undef TSB_ATTN_LAUNCH
 }
 
-int attn_prompt_splits(int max_len) { return attn_split_merge_mode() ? (max_len + attn_prompt_chunk(max_len) - 1) / attn_prompt_chunk(max_len) : MAX_SPLITS; }
+int attn_prompt_splits(int max_len, int prompt_chunk) { return attn_split_merge_mode() ? (max_len + prompt_chunk - 1) / prompt_chunk : MAX_SPLITS; }
 
 extern "C" {
 

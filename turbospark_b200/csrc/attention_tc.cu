@@ -405,13 +405,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 struct TcPlan {
     int n_qtiles, groups, n_splits, chunk;
 };
-TcPlan attn_tc_plan(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, bool prompt) {
+TcPlan attn_tc_plan(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, int max_len, int prompt_chunk) {
     TcPlan p;
     const int G = n_q_heads / kv->view.kv_heads;
     p.n_qtiles = (rows_per_seq * G + TC_QM - 1) / TC_QM;
     p.groups = rows / rows_per_seq;
-    if (prompt) {
-        p.chunk = attn_prompt_chunk(max_len), p.n_splits = attn_prompt_splits(max_len);
+    if (prompt_chunk > 0) {
+        p.chunk = prompt_chunk, p.n_splits = attn_prompt_splits(max_len, prompt_chunk);
         return p;
     }
     const int planned = max_len > 0 ? (max_len + 511) / 512 * 512 : 512;
@@ -484,7 +484,7 @@ cudaError_t tc_kv_map(const KvView& v, int box_rows, CUtensorMap* out) {
 
 }  // namespace
 
-bool attn_tc_applicable(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads) {
+bool attn_tc_applicable(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows_per_seq, int n_q_heads, bool prompt) {
     static int enabled = -1, min_queries = 65;  // TSB_ATTN_TC=0 keeps every pass on the mma.sync kernel (experiments)
     if (enabled < 0) {
         const char* env = getenv("TSB_ATTN_TC");
@@ -496,7 +496,8 @@ bool attn_tc_applicable(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows
     // the tensor copies take whole boxes of a page: pages of 8, 16, ... token rows, all rows of the pool within 32-bit coordinates
     const int pt = kv->view.page_tokens;
     if (pt < 8 || (pt & (pt - 1)) != 0 || (int64_t)kv->view.layers * 2 * kv->view.num_pages * pt >= (int64_t)1 << 31) return false;
-    if (rows_per_seq * (n_q_heads / kv->view.kv_heads) >= min_queries) return true;
+    // a prompt's last group may have a single row, which has to come out as it would in a full one
+    if (prompt || rows_per_seq * (n_q_heads / kv->view.kv_heads) >= min_queries) return true;
     // few queries per stream but many streams: when streams x kv heads fill the device, a CTA per SM that streams its K/V
     // through tensor copies is the faster one (64 streams x 6 rows at context 4096: 262 vs 316 us per layer); below
     // that the few-query kernel wins, whose smaller CTAs overlap the neighbouring matmuls' prologues
@@ -505,8 +506,8 @@ bool attn_tc_applicable(const tsb_ctx* ctx, const tsb_kv* kv, int rows, int rows
 
 cudaError_t launch_attn_tc_partials(tsb_ctx* ctx, cudaStream_t st, tsb_kv* kv, int layer, const __half* q, int64_t q_stride,
                                     const tsb_row_desc* rows_dev, int rows, int rows_per_seq, int n_q_heads, float scale, int max_len,
-                                    void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, bool prompt) {
-    const TcPlan p = attn_tc_plan(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt);
+                                    void* scratch, const float** part_o_out, const float2** part_ml_out, int* n_splits_out, int prompt_chunk) {
+    const TcPlan p = attn_tc_plan(ctx, kv, rows, rows_per_seq, n_q_heads, max_len, prompt_chunk);
     float* part_o = reinterpret_cast<float*>(scratch);
     float2* part_ml = reinterpret_cast<float2*>(part_o + (size_t)rows * n_q_heads * p.n_splits * TC_HD);
     *part_o_out = part_o, *part_ml_out = part_ml, *n_splits_out = p.n_splits;

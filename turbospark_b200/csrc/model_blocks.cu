@@ -546,16 +546,17 @@ static cudaError_t forward_device_wide(tsb_session* s, ModelRt& rt, const int32_
     // A prompt's groups attend like streams of one pass - a group sees the ones before it as committed rows, which the launch before
     // has just written - as many at a time as their shares fit the scratch; the last, shorter one on its own.
     auto attend_prompt = [&](int L, int64_t qkv_dim) -> cudaError_t {
+        const int chunk = attn_prompt_chunk(c.max_context);
         for (int r0 = 0; r0 < rows;) {
             const int per = std::min(PROMPT_GROUP, rows - r0);
             int groups = (rows - r0) / per;
-            auto shares = [&](int g) { return (int64_t)g * per * attn_prompt_splits(max_len); };
+            auto shares = [&](int g) { return (int64_t)g * per * attn_prompt_splits(max_len, chunk); };
             const int64_t room = (int64_t)(rt.attn_scratch_bytes / ((size_t)c.n_q_heads * (c.head_dim + 2) * sizeof(float)));
             while (groups > 1 && shares(groups) > room) groups = (groups + 1) / 2;
             ActOut group = next;
             group.row0 = r0;
             cudaError_t e = launch_attn_decode_rows(ctx, st, rt.kv, L, rt.w_qkv + r0 * qkv_dim, qkv_dim, nullptr, group, rows_dev + r0,
-                                                    groups * per, per, c.n_q_heads, scale, max_len, rt.attn_scratch, rt.attn_rows, true);
+                                                    groups * per, per, c.n_q_heads, scale, max_len, rt.attn_scratch, rt.attn_rows, chunk);
             if (e != cudaSuccess) return e;
             r0 += groups * per;
         }
