@@ -65,6 +65,7 @@ struct TcBars {
     uint64_t kv_full[TC_STAGES], kv_empty[TC_STAGES];
     uint64_t s_full[2], p_full[2], mx_full[2];
     uint64_t pv_full, fin_full;
+    uint64_t mma_over;  // every MMA that was issued has finished
     uint32_t tmem_base, failed;
 };
 
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (threadIdx.x == 0) {
         for (int i = 0; i < TC_STAGES; i++) mbar_init(&bars->kv_full[i], 1), mbar_init(&bars->kv_empty[i], 1);
         for (int i = 0; i < 2; i++) mbar_init(&bars->s_full[i], 1), mbar_init(&bars->p_full[i], TC_SOFTMAX_WARPS), mbar_init(&bars->mx_full[i], TC_SOFTMAX_WARPS);
-        mbar_init(&bars->pv_full, 1), mbar_init(&bars->fin_full, TC_SOFTMAX_WARPS);
+        mbar_init(&bars->pv_full, 1), mbar_init(&bars->fin_full, TC_SOFTMAX_WARPS), mbar_init(&bars->mma_over, 1);
         bars->failed = 0;
         mbar_fence_init();
     }
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         // page of the stream's last position, so that no stale shared memory meets the tensor core.
         if (lane == 0) {
             bool ok = true;
+            int issued = 0;
             const int64_t rows_per_plane = (int64_t)kv.num_pages * kv.page_tokens;  // token rows of one layer's K (or V)
             for (int tile = 0; tile < n_tiles && ok; tile++) {
                 const int st = tile % TC_STAGES;
@@ -185,8 +187,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                         tc_tensor_g2s_2d(vdst + b * (TC_TN * 128) + off, &kvmap, kvh * TC_HD + b * 64, (int)row_v, &bars->kv_full[st]);
                     }
                 }
+                issued = tile + 1;
             }
             if (!ok) bars->failed = 1;
+            // no copy is in flight when the CTA leaves, also when another role has given up
+            for (int t = issued > TC_STAGES ? issued - TC_STAGES : 0; t < issued; t++) mbar_wait(&bars->kv_full[t % TC_STAGES], (t / TC_STAGES) & 1, err);
         }
     } else if (warp == TC_SOFTMAX_WARPS + TC_LOAD_WARPS) {
         // ---- MMA issue: one thread walks the tiles
@@ -243,6 +248,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 TTRC(t, 2);
             }
             if (!ok) bars->failed = 1;
+            tc_commit(&bars->mma_over);  // nor is an MMA when tensor memory is given back
+            mbar_wait(&bars->mma_over, 0, err);
         }
         __syncwarp();
     } else {

@@ -79,6 +79,7 @@ struct WideBars {
     uint64_t a_full[2][2], a_empty[2][2];
     uint64_t d_full[2];  // a block's accumulators are complete
     uint64_t scale_full[WIDE_SCALE_SLOTS];
+    uint64_t mma_over;   // every MMA that was issued has finished
     uint32_t tmem_base;
     uint32_t failed;
     uint32_t ticket;
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             mbar_init(&bars->d_full[i], 1);
         }
         for (int i = 0; i < WIDE_SCALE_SLOTS; i++) mbar_init(&bars->scale_full[i], 4);
+        mbar_init(&bars->mma_over, 1);
         bars->failed = 0;
         mbar_fence_init();
     }
@@ -248,6 +250,9 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                     }
                 }
                 if (!ok) bars->failed = 1;
+                // no copy is in flight when the CTA leaves, also when another role has given up
+                for (uint32_t k = nb > WIDE_RAW_STAGES ? nb - WIDE_RAW_STAGES : 0; k < nb; k++)
+                    mbar_wait(&bars->raw_full[k % WIDE_RAW_STAGES], (k / WIDE_RAW_STAGES) & 1, err);
             }
         } else if (warp == WIDE_WARP_ACT) {
             // ---- producer of the activation chunks: its own warp, so a full activation ring never holds up the weights
@@ -266,6 +271,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                     }
                 }
                 if (!ok) bars->failed = 1;
+                for (uint32_t k = nb > n_bst ? nb - n_bst : 0; k < nb; k++) mbar_wait(&bars->b_full[k % n_bst], (k / n_bst) & 1, err);
             }
         } else if (warp == WIDE_WARP_MMA) {
             // ---- MMA issue: one thread walks the blocks
@@ -314,6 +320,8 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                     }
                 }
                 if (!ok) bars->failed = 1;
+                tc_commit(&bars->mma_over);  // nor is an MMA when tensor memory is given back
+                mbar_wait(&bars->mma_over, 0, err);
             }
             __syncwarp();
         }
