@@ -338,22 +338,25 @@ def test_rows_counted_by_value_match_the_oracle(ctx, oracle, vocab, batch, kind)
         tgt[:] = -1.5
     drf = np.roll(tgt[:, :k], 1, axis=2)
     t16, d16 = oracle.f32_to_f16_bits(tgt), oracle.f32_to_f16_bits(drf)
-    checked = 0
     for shape in (dict(temperature=1.0), dict(temperature=0.0), dict(temperature=0.7, top_p=0.8), dict(temperature=1.3, top_k=7, min_p=0.2),
                   dict(temperature=1.0, top_k=200, top_p=0.95)):
         ocfg = oracle.shaping(seed=4, **shape)
         props = rng.integers(0, vocab, size=(batch, k)).astype(np.int32)
+        props[:, 0] = np.argmax(drf[:, 0], axis=1)  # inside every support of the drafter's
         unis = rng.integers(0, 2**63, size=(batch, 2 * k + 1)).astype(np.uint64) * np.uint64(2)
         outs = _run_accept(ctx, oracle, t16, d16, props, unis, **shape)
-        for b in range(min(batch, 3)):
+        checked = 0
+        for b in range(min(batch, 8)):
             acc, toks, draws, margins = oracle.accept_round(t16[b], d16[b], props[b], ocfg, unis[b])
-            # equal probabilities are the rule here, so r * q <= p is often decided within rounding: such rounds say nothing
-            if shape["temperature"] and (margins[0] < 1e-12 or margins[1] < 1e-12):
+            # a round that is decided within rounding says nothing (a margin of zero is not: neither row has the token)
+            if shape["temperature"] and (0.0 < margins[0] < 1e-12 or margins[1] < 1e-12):
                 continue
             checked += 1
+            if shape["temperature"] and np.isfinite(margins[0]):
+                assert abs(outs[b].margin_accept - margins[0]) <= 1e-9 * max(1.0, margins[0]) + 1e-15, (shape, b)
             assert outs[b].status == 0 and outs[b].accepted == acc and outs[b].draws == draws, (shape, b)
             assert list(outs[b].tokens[:acc + 1]) == list(toks), (shape, b, list(outs[b].tokens[:acc + 1]), list(toks))
-    assert checked > 0
+        assert checked > 0, shape
 
 
 @pytest.mark.parametrize("temperature", [1e-310, 3e-3, 10.0, 20.0, 1e4])
