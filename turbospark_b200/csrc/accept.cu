@@ -19,12 +19,14 @@
 // a pre-pass writes the penalised rows as f32 and the same kernels run over them
 // with 32-bit order keys.
 //
-// Parallel layout: one thread-block cluster of eight CTAs per logits row
-// (statistics) or per stream (decision + draw).  Each CTA owns a contiguous
-// eighth of the vocabulary, keeps its f64 exponentials / fixed-point masses in
-// its own shared memory, and the eight CTAs reduce and broadcast through
-// distributed shared memory in a fixed rank order.  Everything a draw needs
-// stays on chip: the logits are read from HBM/L2 once or twice per row.
+// Parallel layout: one thread-block cluster per logits row (statistics) or per
+// stream (decision + draw).  Each CTA owns a contiguous part of the vocabulary,
+// and the CTAs reduce and broadcast through distributed shared memory in a fixed
+// order.  f16 rows: two, four or eight CTAs count their entries by value in
+// shared memory, and sums and cuts run over occupied values
+// (accept_stats_half_kernel).  f32 rows, decisions and draws: eight CTAs, which
+// keep their f64 exponentials / fixed-point masses there, entry by entry.  The
+// logits are read from HBM/L2 once or twice per row.
 #include <cooperative_groups.h>
 
 #include "accept.cuh"
@@ -359,10 +361,10 @@ __device__ void cluster_find_cut(cg::cluster_group& cluster, DrawShared& c, cons
 }
 
 // ---------------------------------------------------------------- statistics
-// One cluster per row: max / first argmax / finiteness, sum_i exp(l_i - max), total = sum_i w_i.
-template <typename LT, bool HOT>
+// One cluster per f32 row: max / first argmax / finiteness, sum_i exp(l_i - max), total = sum_i w_i.
+template <bool HOT>
 __global__ void __launch_bounds__(ACC_THREADS)
-    accept_stats_kernel(const LT* __restrict__ target, const LT* __restrict__ draft, int k, int vocab,
+    accept_stats_kernel(const float* __restrict__ target, const float* __restrict__ draft, int k, int vocab,
                         double temperature, TruncShape tr, RowStats* __restrict__ stats, int rows_per_stream) {
     extern __shared__ __align__(16) uint8_t dyn[];
     double* ecache = reinterpret_cast<double*>(dyn);  // exp(l - max) of this CTA's slice
@@ -378,8 +380,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
     pdl_wait();
     const int b = row_id / rows_per_stream, r = row_id % rows_per_stream;
     // rows 0..k are the target's, k+1..2k the drafter's
-    const LT* row = (r <= k) ? target + ((size_t)b * (k + 1) + r) * vocab
-                                  : draft + ((size_t)b * k + (r - k - 1)) * vocab;
+    const float* row = (r <= k) ? target + ((size_t)b * (k + 1) + r) * vocab : draft + ((size_t)b * k + (r - k - 1)) * vocab;
     const Slice sl = my_slice(vocab, rank);
     if (threadIdx.x == 0) bad_flag = 0;
     __syncthreads();
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
     int am = 0x7fffffff;
     bool bad = false;
     for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS) {
-        const float v = Logit<LT>::val(row[sl.lo + j]);
+        const float v = row[sl.lo + j];
         bad |= !isfinite(v);
         if (v > mx) mx = v, am = sl.lo + j;  // indices grow with j, so the first maximum is kept
     }
@@ -419,12 +420,12 @@ __global__ void __launch_bounds__(ACC_THREADS)
     cluster.sync();
     RowStats st;
     st.max = mx, st.argmax = am, st.sum = 1.0, st.total = 1.0, st.nonfinite = nonfinite;
-    st.has_cut = 0, st.cut_key = Logit<LT>::KEY_MAX, st.cut_idx = 0x7fffffff, st.min_e = 0.0;
+    st.has_cut = 0, st.cut_key = Logit<float>::KEY_MAX, st.cut_idx = 0x7fffffff, st.min_e = 0.0;
     if (temperature != 0.0 && !nonfinite) {
         const double dmx = (double)mx;
         double s = 0.0;
         for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS) {
-            const double e = exp((double)Logit<LT>::val(row[sl.lo + j]) - dmx);
+            const double e = exp((double)row[sl.lo + j] - dmx);
             ecache[j] = e;
             s += e;
         }
@@ -433,11 +434,11 @@ __global__ void __launch_bounds__(ACC_THREADS)
         const bool unit_t = temperature == 1.0;
         st.sum = sum;
         const bool truncating = (tr.top_k > 0 && tr.top_k < (unsigned)vocab) || tr.top_p > 0.0 || tr.min_p > 0.0;
-        if (truncating) cluster_find_cut<LT>(cluster, c, ecache, sum, row, sl, vocab, tr, &st);
+        if (truncating) cluster_find_cut<float>(cluster, c, ecache, sum, row, sl, vocab, tr, &st);
         double t = 0.0;
         for (int j = threadIdx.x; j < sl.n; j += ACC_THREADS)
             if (!truncating || survives_e(st, row[sl.lo + j], sl.lo + j, ecache[j]))
-                t += unit_t ? ecache[j] : weight_of<HOT>((double)Logit<LT>::val(row[sl.lo + j]) - dmx, inv_t, unit_t, sum);
+                t += unit_t ? ecache[j] : weight_of<HOT>((double)row[sl.lo + j] - dmx, inv_t, unit_t, sum);
         st.total = cluster_sum_f64(cluster, &xch, 1, block_sum_f64(t, red));
     }
     pdl_launch_dependents();
@@ -1220,7 +1221,7 @@ cudaError_t configure_kernels(const tsb_ctx* ctx) {
     if constexpr (sizeof(LT) == 2)
         e = tsb_opt_in_smem(ctx, accept_stats_half_kernel<HOT>, (size_t)KEYS * 2, stats_done);
     else
-        e = tsb_opt_in_smem(ctx, accept_stats_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, stats_done);
+        e = tsb_opt_in_smem(ctx, accept_stats_kernel<HOT>, (size_t)SLICE_MAX * 8, stats_done);
     if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, accept_decide_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, decide_done);
     if (e == cudaSuccess) e = tsb_opt_in_smem(ctx, sample_kernel<LT, HOT>, (size_t)SLICE_MAX * 8, sample_done);
     return e;
@@ -1318,7 +1319,7 @@ static cudaError_t launch_stats(tsb_ctx* ctx, cudaStream_t st, const LT* target,
         return tsb_launch_cluster(ctx, accept_stats_half_kernel<HOT>, dim3((unsigned)(rows * n)), dim3(ACC_THREADS), (size_t)KEYS * 2, st, true, (unsigned)n, target,
                                   draft, k, vocab, temperature, tr, stats, rows_per_stream);
     } else {
-        return tsb_launch_cluster(ctx, accept_stats_kernel<LT, HOT>, dim3((unsigned)(rows * CL)), dim3(ACC_THREADS), slice_smem(vocab), st, true, (unsigned)CL,
+        return tsb_launch_cluster(ctx, accept_stats_kernel<HOT>, dim3((unsigned)(rows * CL)), dim3(ACC_THREADS), slice_smem(vocab), st, true, (unsigned)CL,
                                   target, draft, k, vocab, temperature, tr, stats, rows_per_stream);
     }
 }

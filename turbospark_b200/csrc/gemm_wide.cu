@@ -86,8 +86,8 @@ struct WideBars {
 };
 
 // x natural [tokens, cols] f16 -> for every pass of `per_pass` token rows and every 256-column block, n_pad tokens x 34 chunks
-// of 16 bytes (see the file header); pass p starts at p * units * 34 * per_pass chunks and its own n_pad is its
-// token count rounded up to 16.  A CTA takes eight tokens of one block: warp = token, lane = 16-byte chunk; the
+// of 16 bytes (see the file header); n_pad is per_pass for every pass, the last one's missing rows being zeros, so that pass p
+// starts at p * units * 34 * per_pass chunks.  A CTA takes eight tokens of one block: warp = token, lane = 16-byte chunk; the
 // 32-column sums come from two shuffles over the four lanes of a sub-block; the CTA's 34 x 8 chunks go out through
 // shared memory as 128-byte runs.
 __global__ void __launch_bounds__(256) wide_prepare_kernel(const __half* __restrict__ x, int64_t x_stride, int tokens, int per_pass, int units,
@@ -436,18 +436,18 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                         }
                 } else {
 #pragma unroll
-                for (int c = 0; c < ROUNDS; c += 2)
-                    if (16 * c < cpw) {
-                        uint32_t v0[16], v1[16];
-                        tc_ld16(from + col0 + 16 * c, v0);
-                        tc_ld16(from + col0 + 16 * c + 16, v1);
-                        tc_wait_ld(v0, v1);
+                    for (int c = 0; c < ROUNDS; c += 2)
+                        if (16 * c < cpw) {
+                            uint32_t v0[16], v1[16];
+                            tc_ld16(from + col0 + 16 * c, v0);
+                            tc_ld16(from + col0 + 16 * c + 16, v1);
+                            tc_wait_ld(v0, v1);
 #pragma unroll
-                        for (int i = 0; i < 16; i++) {
-                            acc[16 * c + i] = fmaf(by, __uint_as_float(v0[i]), acc[16 * c + i]);
-                            acc[16 * c + 16 + i] = fmaf(by, __uint_as_float(v1[i]), acc[16 * c + 16 + i]);
+                            for (int i = 0; i < 16; i++) {
+                                acc[16 * c + i] = fmaf(by, __uint_as_float(v0[i]), acc[16 * c + i]);
+                                acc[16 * c + 16 + i] = fmaf(by, __uint_as_float(v1[i]), acc[16 * c + 16 + i]);
+                            }
                         }
-                    }
                 }
                 tc_fence_before();
                 __syncwarp();

@@ -11,8 +11,6 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// D[tmem_d] (+)= A[tmem_a] * B[smem descriptor]; M = 128, K = 16, f16 or bfloat16 inputs, f32 accumulate.  ACC = false overwrites D.
-// tc_issue_ss: A from shared memory (a matrix descriptor like B's).
 // One lane of a converged warp, always the same one.  A thread that this picks issues the instructions and the commits on its own: an MMA whose
 // predicate differs between the lanes of a converged warp took 75 to 90 cycles to issue, one from a single thread about 25.
 __device__ __forceinline__ bool tc_elect() {
@@ -26,6 +24,8 @@ __device__ __forceinline__ bool tc_elect() {
         : "=r"(one));
     return one != 0;
 }
+// D[tmem_d] (+)= A[tmem_a] * B[smem descriptor]; M = 128, K = 16, f16 or bfloat16 inputs, f32 accumulate.  ACC = false overwrites D.
+// tc_issue_ss: A from shared memory (a matrix descriptor like B's).
 template <bool ACC>
 __device__ __forceinline__ void tc_issue_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc) {
     asm volatile(
