@@ -831,3 +831,21 @@ def test_a_prompts_rows_do_not_depend_on_the_rows_behind_them(long_rig, short, l
         got.append(sess.produce(int(tokens[at]), at).copy())
     sess.close()
     assert np.array_equal(got[0], got[1])
+
+
+def test_rounds_captured_at_a_high_temperature_equal_enqueued_ones(rig):
+    """Sampling above a temperature of ten has kernels of its own: a session that has sampled below it captures them in its next round."""
+    tsb = rig["tsb"]
+    K, streams, got = 3, 2, []
+    for graph in (True, False):
+        sess = tsb.Session(rig["ctx"], rig["target"], rig["draft"], streams, 8)
+        sess.set_graph(graph)
+        sess.fill_context(40, seed=3)
+        nxt, steps, toks = np.array([5, 900], dtype=np.int32), np.zeros(streams, dtype=np.uint64), []
+        for temperature in (1.0, 20.0, 20.0, 20.0, 1.0):
+            rc = tsb.run_config(tsb.shaping(temperature=temperature, seed=2), 64, K, uniform_mode=1)
+            accepted, committed = sess.round_tokens(rc, nxt, steps)
+            toks.append((list(accepted), committed.tolist(), list(nxt)))
+        got.append(toks)
+        sess.close()
+    assert got[0] == got[1]
