@@ -81,7 +81,7 @@ constexpr int gemm_ctas_per_sm() {
     return NT == 1 && QT == TSB_Q4_K ? TSB_GEMM_CTAS_NT1 : (NT <= 2 ? 2 : 1);
 }
 
-template <int QT, int NT, int EPI, bool GROUPED = false>
+template <int QT, int NT, int EPI, bool GROUPED = false, bool PACK = false>
 __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
     gemm_quant_kernel(const uint8_t* __restrict__ W0, int64_t rows, int units /*256-col units per row*/,
                       ActOperand act, int tokens, int tok0, EpiArgs epi, uint32_t* __restrict__ err, GroupedArgs grp) {
@@ -112,17 +112,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
 #endif
     GTRC(0);
     const int n_tiles = (int)((rows + TILE_ROWS - 1) / TILE_ROWS);
-    // Narrow expert matrices: a row of `units` < 8 blocks gives work to that many of the eight consumer warps, so a stage holds
-    // the same row range's neighbours too - `pack` row tiles side by side, a tile's rows `region` bytes behind its
+    // PACK, for narrow expert matrices: a row of at most four blocks gives work to that many of the eight consumer warps, so a stage
+    // holds the same row range's neighbours too - `pack` row tiles side by side, a tile's rows `region` bytes behind its
     // neighbour's - and `units` warps take each.  (The down projections of 128 MXFP4 experts, 2048 x 768, three units: one tile a
     // stage kept five warps idle and paid a stage's hand-shake, barrier and store for 6.5 KB of weights: the routed feed-forward of
-    // 40 rows takes 184 us where it took 202; 64 rows over 1024 x 256, one unit, 76 where it took 95.)
+    // 40 rows takes 177 us where it took 200; 64 rows over 1024 x 256, one unit, 75 where it took 94.)
     // How many: an item costs its tiles plus about one tile's time, and the items go to the CTAs in waves, so the cheapest number of
     // tiles is small where few experts have rows.  (Always as many as fit, two experts of 64 tiles and one unit were 20 items of seven
-    // tiles for 296 CTAs: that feed-forward took 15.7 us where one tile a stage takes 12.6; by this rule 12.9.)
-    constexpr bool CAN_PACK = GROUPED && EPI == EPI_PLAIN;
+    // tiles for 296 CTAs: that feed-forward took 15.2 us where one tile a stage takes 12.3; by this rule 12.3 to 12.7.)
+    // Wider rows fill the warps by themselves and keep the kernel without: with this code in theirs a token of two 2048 x 2048 MXFP4 experts took 18.9 us instead of 17.3.
+    static_assert(!PACK || (GROUPED && EPI == EPI_PLAIN), "packed tiles");
     const int region = (units * UB + 30) & ~15;
-    const int most = CAN_PACK && 2 * units <= STAGE_UNITS ? min(STAGE_UNITS / units, ROW_STRIDE / region) : 1;
     const int iters = (units + STAGE_UNITS - 1) / STAGE_UNITS;  // stages per row tile
     const int64_t row_bytes = (int64_t)units * UB;
 
@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
                 base += __popc(mask);
             }
             if (lane == 0) grp_active = base;
-            if constexpr (CAN_PACK) {  // lane l: the cost of l + 1 tiles
+            if constexpr (PACK) {  // lane l: the cost of l + 1 tiles
+                const int most = min(STAGE_UNITS / units, ROW_STRIDE / region);
                 const int waves = (base * ((n_tiles + lane) / (lane + 1)) + (int)gridDim.x - 1) / (int)gridDim.x;
                 const uint32_t cost = lane < most ? (uint32_t)waves * (uint32_t)(lane + 2) : 0x7FFFFFFu;
                 const uint32_t best = __reduce_min_sync(0xffffffffu, min(cost, 0x7FFFFFFu) << 5 | (uint32_t)lane);
@@ -161,9 +162,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
         }
     }
     __syncthreads();
-    int pack = 1;
-    if constexpr (CAN_PACK) pack = grp_pack;
-    const int n_groups = CAN_PACK ? (n_tiles + pack - 1) / pack : num_groups<EPI>(n_tiles, epi);
+    const int pack = PACK ? grp_pack : 1;
+    const int n_groups = PACK ? (n_tiles + pack - 1) / pack : num_groups<EPI>(n_tiles, epi);
     const int n_items = GROUPED ? n_groups * grp_active : n_groups;
 
     // The CTA is persistent: it walks groups blockIdx.x, +gridDim.x, ... and the stage ring runs on across
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
                 g = item - a * n_groups;
                 W = W0 + (int64_t)grp_mat[a] * grp.w_stride;
             }
-            if (CAN_PACK && pack > 1) {
+            if constexpr (PACK) {
                 const uint32_t s = n % NUM_STAGES;
                 if (n >= NUM_STAGES && !mbar_wait(&empty[s], ((n / NUM_STAGES) - 1) & 1, err)) return;
                 n++;
@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
             }
         }
         Group gr = group_of<EPI>(g, n_tiles, epi);
-        const int sub = CAN_PACK && pack > 1 ? warp / units : 0;  // this warp's tile of the group
-        if (CAN_PACK && pack > 1) gr.tile0 = g * pack;
+        const int sub = PACK ? warp / units : 0;  // this warp's tile of the group
+        if (PACK) gr.tile0 = g * pack;
         // finished tiles alternate between two buffers, so a group's epilogue may still be reading its tiles while
         // the next group's sums are written: no barrier after the epilogue
         float* tile_out = tile_out0 + (group_no++ & 1u) * (2 * NTOK * 16);
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
                 if (n == 0) { GTRC(2); }
                 const int nun = min(STAGE_UNITS, units - it * STAGE_UNITS);
                 const int wu = warp - sub * units;  // this warp's block of the row
-                if (ok && (CAN_PACK && pack > 1 ? sub < pack && row0 < rows : warp < nun)) {
+                if (ok && (PACK ? sub < pack && row0 < rows : warp < nun)) {
                     // slack of this stage's source address: the row start's slack plus the stage offset
                     const uint32_t stA = ALIGNED_ROWS ? 0u : (slackA + (uint32_t)((int64_t)it * STAGE_UNITS * UB)) & 15u;
                     const uint32_t stB = ALIGNED_ROWS ? 0u : (slackB + (uint32_t)((int64_t)it * STAGE_UNITS * UB)) & 15u;
@@ -344,14 +344,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
             if (!ELEMWISE && ti + 1 < gr.n) continue;  // the pair's second tile first
             epilogue_prefetch<EPI, NT>(epi, gr, rows, tokens, tok0);
             asm volatile("bar.sync 1, %0;" ::"n"(CONSUMER_WARPS * 32) : "memory");
-            if (CAN_PACK && pack > 1) {
+            if constexpr (PACK) {
                 // tile by tile, the sums in the order of the blocks; the thread that sums an element stores it
                 for (int t = 0; t < pack && gr.tile0 + t < n_tiles; t++) {
                     for (int idx = threadIdx.x; idx < NTOK * 16; idx += CONSUMER_WARPS * 32) {
                         const int tok = idx >> 4, row = idx & 15, nn = tok & 7;
                         const float* p = redb + ((t * units * NT + (tok >> 3)) * 4 + (((row >> 3) << 1) | (nn & 1))) * 32 + (row & 7) * 4 + (nn >> 1);
                         float sum = 0.f;
-                        for (int w = 0; w < units; w++) sum += p[w * NT * 4 * 32];
+#pragma unroll
+                        for (int w = 0; w < STAGE_UNITS / 2; w++)
+                            if (w < units) sum += p[w * NT * 4 * 32];
                         tile_out[idx] = sum;
                     }
                     if (ok) run_epilogue<EPI, NT>(epi, Group{gr.tile0 + t, 0, 1}, tile_out, inv_rms, rows, tokens, tok0, err);
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, (gemm_ctas_per_sm<QT, NT>()))
         }
         // (run_epilogue reads tile_out[idx] with the same idx -> thread mapping as the sum loop: no barrier between)
         if (item == (int)blockIdx.x) { GTRC(4); }
-        if (ok && !(CAN_PACK && pack > 1)) run_epilogue<EPI, NT>(epi, gr, tile_out, inv_rms, rows, tokens, tok0, err);
+        if (ok && !PACK) run_epilogue<EPI, NT>(epi, gr, tile_out, inv_rms, rows, tokens, tok0, err);
         if (item == (int)blockIdx.x) { GTRC(5); }
     }
     GTRC(6);
@@ -398,10 +400,10 @@ constexpr size_t gemm_smem_bytes() {
            (size_t)NUM_STAGES * TILE_ROWS * row_stride_for(Fmt<QT>::UNIT_BYTES) + 128;
 }
 
-template <int QT, int NT, int EPI, bool GROUPED = false>
+template <int QT, int NT, int EPI, bool GROUPED = false, bool PACK = false>
 cudaError_t launch_one(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t rows, int units, ActOperand act, int tokens,
                        int tok0, const EpiArgs& args, const GroupedArgs& grp = GroupedArgs()) {
-    auto kern = gemm_quant_kernel<QT, NT, EPI, GROUPED>;
+    auto kern = gemm_quant_kernel<QT, NT, EPI, GROUPED, PACK>;
     static SmemOptIn configured;  // per instantiation and per device
     constexpr size_t smem = gemm_smem_bytes<QT, NT>();
     if (cudaError_t e = tsb_opt_in_smem(ctx, kern, smem, configured); e != cudaSuccess) return e;
@@ -426,20 +428,20 @@ cudaError_t launch_one(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t 
 
 // The matrices are binned by their row count, one launch per bin with the token-tile width that fits it: a matrix
 // with three rows is not run through the 64-column variant because another one has forty.
-template <int QT, int EPI>
+template <int QT, int EPI, bool PACK>
 cudaError_t launch_grouped_nt(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t rows, int units, ActOperand act, int max_tokens,
                               const EpiArgs& args, GroupedArgs grp) {
     cudaError_t e;
     grp.chunk0 = 0, grp.lo = 0, grp.hi = 8;
-    if ((e = launch_one<QT, 1, EPI, true>(ctx, st, w, rows, units, act, 8, 0, args, grp)) != cudaSuccess || max_tokens <= 8) return e;
+    if ((e = launch_one<QT, 1, EPI, true, PACK>(ctx, st, w, rows, units, act, 8, 0, args, grp)) != cudaSuccess || max_tokens <= 8) return e;
     grp.lo = 8, grp.hi = 16;
-    if ((e = launch_one<QT, 2, EPI, true>(ctx, st, w, rows, units, act, 16, 0, args, grp)) != cudaSuccess || max_tokens <= 16) return e;
+    if ((e = launch_one<QT, 2, EPI, true, PACK>(ctx, st, w, rows, units, act, 16, 0, args, grp)) != cudaSuccess || max_tokens <= 16) return e;
     grp.lo = 16, grp.hi = 32;
-    if ((e = launch_one<QT, 4, EPI, true>(ctx, st, w, rows, units, act, 32, 0, args, grp)) != cudaSuccess || max_tokens <= 32) return e;
+    if ((e = launch_one<QT, 4, EPI, true, PACK>(ctx, st, w, rows, units, act, 32, 0, args, grp)) != cudaSuccess || max_tokens <= 32) return e;
     grp.lo = 32, grp.hi = 0x7fffffff;
     for (int t0 = 0; t0 < max_tokens; t0 += 64) {
         grp.chunk0 = t0;
-        if ((e = launch_one<QT, 8, EPI, true>(ctx, st, w, rows, units, act, 64, 0, args, grp)) != cudaSuccess) return e;
+        if ((e = launch_one<QT, 8, EPI, true, PACK>(ctx, st, w, rows, units, act, 64, 0, args, grp)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -447,8 +449,9 @@ cudaError_t launch_grouped_nt(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, i
 template <int QT>
 cudaError_t launch_grouped_epi(tsb_ctx* ctx, cudaStream_t st, const uint8_t* w, int64_t rows, int units, ActOperand act, int tokens,
                                int epi, const EpiArgs& args, const GroupedArgs& grp) {
-    if (epi == EPI_MOE_ACT) return launch_grouped_nt<QT, EPI_MOE_ACT>(ctx, st, w, rows, units, act, tokens, args, grp);
-    if (epi == EPI_PLAIN) return launch_grouped_nt<QT, EPI_PLAIN>(ctx, st, w, rows, units, act, tokens, args, grp);
+    if (epi == EPI_MOE_ACT) return launch_grouped_nt<QT, EPI_MOE_ACT, false>(ctx, st, w, rows, units, act, tokens, args, grp);
+    if (epi == EPI_PLAIN && 2 * units <= STAGE_UNITS) return launch_grouped_nt<QT, EPI_PLAIN, true>(ctx, st, w, rows, units, act, tokens, args, grp);
+    if (epi == EPI_PLAIN) return launch_grouped_nt<QT, EPI_PLAIN, false>(ctx, st, w, rows, units, act, tokens, args, grp);
     return cudaErrorInvalidValue;
 }
 
