@@ -472,8 +472,9 @@ static int32_t blocks_runtime_init(tsb_session* s, ModelRt& rt, const tsb_model*
         const char* env = getenv("TSB_WIDE_FORWARD");
         if (env && env[0] == '0') wide = false;
     }
-    // Prompts go through the target in passes of up to PROMPT_ROWS rows there: 1000 tokens of the 8B shape took 71 ms in passes of
-    // 64, whose weights are read and dequantised sixteen times.  Buffers of a pass: 170 MB at that shape.
+    // Prompts go through the target in passes of up to PROMPT_ROWS rows there (or of the session's largest pass, where that has more):
+    // 1000 tokens of the 8B shape took 71 ms in passes of 64, whose weights are read and dequantised sixteen times, and take 25.  The
+    // buffers add 96 MB to a session of 128 rows per pass at that shape, 213 MB to one of 32.
     if (wide && !is_draft) rt.prompt_rows = std::max(R, std::min(PROMPT_ROWS, c.max_context));
     const int W = std::max(R, rt.prompt_rows);  // rows of the buffers a prompt's pass uses
     if ((rc = A((size_t)W * c.d_model * 2, (void**)&rt.h))) return rc;
